@@ -46,18 +46,30 @@ def ours_f64(pkg, view, dp, p, filter_img=False):
 
 
 class RefKernels:
-    """The reference project's runDiff2KernelCoarse / runDiff2KernelCoarseDouble."""
+    """The reference project's runDiff2KernelCoarse / runDiff2KernelCoarseDouble,
+    loaded at first use (a test that uses them is skipped where they were not
+    built, see conftest.skip_without_reference_kernels)."""
 
     def __init__(self, oracle, pr):
-        self.L = oracle.ref_lib()
-        pv = pr.projector
-        re = np.ascontiguousarray(pv.re, np.float32)
-        im = np.ascontiguousarray(pv.im, np.float32)
-        self.h = self.L.refshim_projector_create(pv.mdlX, pv.mdlY, pv.mdlZ, pv.mdlInitY, pv.mdlInitZ,
-                                                 pv.mdlMaxR, pv.padding_factor,
-                                                 re.ctypes.data_as(C.c_void_p), im.ctypes.data_as(C.c_void_p))
-        assert self.h
+        self.oracle = oracle
         self.pr = pr
+        self._h = None
+
+    @property
+    def L(self):
+        return self.oracle.ref_lib()
+
+    @property
+    def h(self):
+        if self._h is None:
+            pv = self.pr.projector
+            re = np.ascontiguousarray(pv.re, np.float32)
+            im = np.ascontiguousarray(pv.im, np.float32)
+            self._h = self.L.refshim_projector_create(pv.mdlX, pv.mdlY, pv.mdlZ, pv.mdlInitY, pv.mdlInitZ,
+                                                      pv.mdlMaxR, pv.padding_factor,
+                                                      re.ctypes.data_as(C.c_void_p), im.ctypes.data_as(C.c_void_p))
+            assert self._h
+        return self._h
 
     def f32(self, dp, p, init=None):
         pr, torch = self.pr, dp.torch
@@ -85,9 +97,9 @@ class RefKernels:
         return out.cpu().numpy().reshape(pr.O, pr.T)
 
     def close(self):
-        if self.h:
-            self.L.refshim_projector_destroy(self.h)
-            self.h = None
+        if self._h:
+            self.L.refshim_projector_destroy(self._h)
+            self._h = None
 
 
 def argmin_consistent(test, ref, rel_tol):
