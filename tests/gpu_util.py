@@ -62,10 +62,11 @@ class RefKernels:
     @property
     def h(self):
         if self._h is None:
+            L = self.L
             pv = self.pr.projector
             re = np.ascontiguousarray(pv.re, np.float32)
             im = np.ascontiguousarray(pv.im, np.float32)
-            self._h = self.L.refshim_projector_create(pv.mdlX, pv.mdlY, pv.mdlZ, pv.mdlInitY, pv.mdlInitZ,
+            self._h = L.refshim_projector_create(pv.mdlX, pv.mdlY, pv.mdlZ, pv.mdlInitY, pv.mdlInitZ,
                                                       pv.mdlMaxR, pv.padding_factor,
                                                       re.ctypes.data_as(C.c_void_p), im.ctypes.data_as(C.c_void_p))
             assert self._h
