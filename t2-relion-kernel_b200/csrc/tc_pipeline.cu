@@ -2276,9 +2276,12 @@ __global__ void __launch_bounds__(GEN ? kGemmThreadsGen : kGemmThreads, 1)
     bool vrow = false;
     EpiRow x;
     if (epi) x = epi_row<C::kScaled>(g, m0 + row, p, vrow);
+    // a CTA that gave up has no sums: its cluster leaves the tile unwritten
+    if (threadIdx.x == 0 && *s_abort)
+      for (int r = 0; r < nsplit; ++r) sm100::st_cluster_u32(sm100::map_to_rank(tmem_slot + 1, (uint32_t)r), 1u);
     __syncthreads();
-    sm100::cluster_sync();  // every part has arrived, and nothing remote follows
-    if (epi) {
+    sm100::cluster_sync();  // every part and flag has arrived, and nothing remote follows
+    if (epi && !*s_abort) {
       float best = __int_as_float(0x7f800000);
       int best_lo = -1;
       if (vrow) {

@@ -1,0 +1,65 @@
+"""Give-up paths: when a bounded device-side wait runs out, nothing that depends
+on it is stored.  The limit is cut by the test hook; the kernels drain what
+they have in flight and return, the status reads B200D2_ERR_TIMEOUT, and the
+next call with the default limit is correct in the same workspace.
+
+Scores that were written all the same must be the right ones: 1e-5 relative
+against the FP64 kernel, plus 6e-8 for the addition onto the initial value."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from gpu_util import DeviceProblem
+
+pytestmark = pytest.mark.gpu
+TIMEOUT = 5  # B200D2_ERR_TIMEOUT
+
+
+@pytest.fixture(scope="module")
+def c2(pkg, synth, cuda):
+    pr = synth.make_problem("c2", P=2)
+    proj = pkg.Projector(pr.projector, use_texture=1)
+    view = proj.view(pr.imgX, pr.imgY, pr.imgMaxR)
+    dp = DeviceProblem(cuda, pr)
+    ref = []
+    for p in range(pr.P):
+        d = cuda.zeros(pr.O * pr.T, device="cuda", dtype=cuda.float64)
+        pkg.run_diff2_kernel_coarse_double(view, dp.tx, dp.ty, dp.corr[p], dp.re[p], dp.im[p], dp.eulers, d, pr.O,
+                                           pr.T, pr.N_img)
+        ref.append(d)
+    yield pr, view, dp, cuda.stack(ref).reshape(pr.P, pr.O, pr.T)
+    proj.close()
+
+
+@pytest.mark.parametrize("split", [2, 3, 8])
+def test_split_tile_that_gave_up_is_not_written(pkg, cuda, c2, split):
+    """A 1 us limit runs out in the epilogue's wait for the accumulator (tens of
+    k-blocks per CTA of the cluster): added scores stay as they were."""
+    torch = cuda
+    pr, view, dp, ref = c2
+    init = (2.0 ** torch.floor(torch.log2(ref))).float()  # of the score's size: the sum rounds once more
+    out = init.clone()
+    b = pkg.make_batch(dp.eulers, dp.tx, dp.ty, dp.re, dp.im, dp.corr, out, O=pr.O, T=pr.T, P=pr.P, N_img=pr.N_img,
+                       accumulate=True)
+    ws = torch.empty(pkg.batch_workspace_bytes(view, b, pkg.PREC_BF16X3), device="cuda", dtype=torch.uint8)
+    pkg.set_gemm_variant(128, 128, split, 2)
+    try:
+        pkg.set_wait_limit_ns(1000)
+        try:
+            pkg.diff2_coarse_batch(view, b, pkg.PREC_BF16X3, ws)
+            torch.cuda.synchronize()
+        finally:
+            pkg.set_wait_limit_ns(0)
+        assert pkg.workspace_status(ws) == TIMEOUT
+        untouched = out == init
+        want = ref + init.double()
+        good = (out.double() - want).abs() <= (1e-5 + 6e-8) * want
+        assert bool((untouched | good).all()) and bool(untouched.any())
+        out.copy_(init)
+        pkg.diff2_coarse_batch(view, b, pkg.PREC_BF16X3, ws)
+        torch.cuda.synchronize()
+        assert pkg.workspace_status(ws) == 0
+        assert ((out.double() - want).abs() / want).max().item() <= 1e-5 + 6e-8
+    finally:
+        pkg.set_gemm_variant(0, 0, 0, 0)
