@@ -563,8 +563,10 @@ int b200d2_set_combine(int mode);
  * partial sums are added in split order in FP64), pair = 1 for CTA-pair tiles
  * (a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs;
  * 256-wide, no k-splits), 2 for single-CTA tiles.  0 in any field restores the
- * default (64-byte rows, 256-wide tiles, k-splits chosen from the tile count, CTA
- * pairs when the pair tiles fill the GPU).  Plans
+ * default (256-wide tiles, CTA pairs when the pair tiles fill the GPU, 128-wide
+ * tiles when those fit in one wave; 128-byte rows for CTA pairs and 128-wide
+ * tiles, else 64-byte rows; k-splits chosen from the tile count).  The server
+ * never splits, so that a request's sums do not depend on its company.  Plans
  * created with B200D2_PLAN_AUTOTUNE choose their own variant; other plans take
  * this setting at creation (single-CTA 256-wide tiles when it is 0). */
 int b200d2_set_gemm_variant(int row_bytes, int tile_n, int split, int pair);

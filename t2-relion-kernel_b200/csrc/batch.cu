@@ -22,7 +22,7 @@ int minloc(const float* d, long long n, int P, double* mn, long long* arg, cudaS
 size_t tc_workspace_bytes(const b200d2_view& view, const b200d2_batch& b, int precision, bool reserve = true);
 int tc_run(const b200d2_view& view, const b200d2_batch& b, int precision, void* ws,
            size_t ws_bytes, cudaStream_t s, const int* d_proj_need = nullptr,
-           float* d_eul_cache = nullptr);
+           float* d_eul_cache = nullptr, bool served = false);
 bool tc_projection_layout(const b200d2_view& v, const b200d2_batch& b, int precision, std::vector<uint64_t>& key);
 
 static int validate(const b200d2_view* v, const b200d2_batch* b) {
@@ -211,9 +211,11 @@ extern "C" size_t b200d2_diff2_coarse_batch_workspace(const b200d2_view* view,
   return b200d2::tc_workspace_bytes(*view, *batch, precision);
 }
 
-extern "C" int b200d2_diff2_coarse_batch(const b200d2_view* view, const b200d2_batch* batch,
-                                         int precision, void* d_workspace,
-                                         size_t workspace_bytes, void* stream) {
+namespace b200d2 {
+// The batch entry point; served: a request of the serving loop, whose sums
+// must not depend on the batch they are taken in (TcGeom::served).
+int batch_run(const b200d2_view* view, const b200d2_batch* batch, int precision, void* d_workspace,
+              size_t workspace_bytes, void* stream, bool served) {
   int st = b200d2::validate(view, batch);
   if (st != B200D2_OK) return st;
   const b200d2_batch& b = *batch;
@@ -236,9 +238,16 @@ extern "C" int b200d2_diff2_coarse_batch(const b200d2_view* view, const b200d2_b
   if (b200d2::is_tc_precision(precision)) {
     const size_t need = b200d2::tc_workspace_bytes(*view, b, precision);
     if (need > 0 && (!d_workspace || workspace_bytes < need)) return B200D2_ERR_INVALID;
-    return b200d2::tc_run(*view, b, precision, d_workspace, workspace_bytes, s);
+    return b200d2::tc_run(*view, b, precision, d_workspace, workspace_bytes, s, nullptr, nullptr, served);
   }
   return B200D2_ERR_UNSUPPORTED;
+}
+}  // namespace b200d2
+
+extern "C" int b200d2_diff2_coarse_batch(const b200d2_view* view, const b200d2_batch* batch,
+                                         int precision, void* d_workspace,
+                                         size_t workspace_bytes, void* stream) {
+  return b200d2::batch_run(view, batch, precision, d_workspace, workspace_bytes, stream, false);
 }
 
 namespace b200d2 {

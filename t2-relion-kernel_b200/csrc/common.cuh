@@ -239,6 +239,11 @@ __host__ __device__ __forceinline__ bool pixel_maybe_inside(int x, int y,
   return r2 < (double)maxR2_padded + 2.0;
 }
 
+// b200d2_diff2_coarse_batch; served: for the serving loop, every sum in the
+// order that a merged batch takes it (batch.cu).
+int batch_run(const b200d2_view* view, const b200d2_batch* batch, int precision, void* d_workspace,
+              size_t workspace_bytes, void* stream, bool served);
+
 // Merged batches: several requests on one reference in one stream-ordered
 // pipeline run, each request's particles against its own orientation columns
 // (tc_pipeline.cu; used by the serving loop).

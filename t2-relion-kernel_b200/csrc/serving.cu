@@ -303,7 +303,7 @@ int admit(b200d2_server* s, Req& q) {
   b.d_min = reinterpret_cast<double*>(d + o_mn);
   b.d_argmin = reinterpret_cast<long long*>(d + o_am);
   const double t_run = now_s();
-  int rc = b200d2_diff2_coarse_batch(&ref.view, &b, s->prec, q.ws_bytes ? d + o_ws : nullptr, q.ws_bytes, st);
+  int rc = b200d2::batch_run(&ref.view, &b, s->prec, q.ws_bytes ? d + o_ws : nullptr, q.ws_bytes, st, true);
   s->st.admit_launch_max_s = std::max(s->st.admit_launch_max_s, now_s() - t_run);
   for (const Down& w : downs) {
     if (!w.dst) continue;

@@ -73,6 +73,10 @@ struct TcGeom {
   // compacted weights hold corr in FP32 at row * Kq floats, the others corr / 2
   // in FP64 at row * Kq doubles (the float rows end before the double rows begin).
   int fused;
+  // a run of the serving loop: every sum in the one order that a request takes
+  // alone and in a merged batch (no k-splits, whose count depends on the batch's
+  // tiles, and the norms by MMAs for few particles too)
+  int served;
   // device flags read by the projection stage (kEulCheckBlocks words): all
   // 0 = the workspace already holds this call's projections (skip the
   // stage), else project and copy the Euler matrices to d_eul_cache; null =
@@ -2883,6 +2887,7 @@ static int launch_gemm_pair(const b200d2_batch& b, const TcGeom& g, void* ws, cu
 template <int PREC>
 static int launch_gemm(const b200d2_batch& b, const TcGeom& g, void* ws, cudaStream_t s, GemmVariant var,
                        const UnevenTabs* U) {
+  if (g.served) var.split = 1;
   if (!U) {  // batch entry points: the process-wide setting fills unset fields
     if (var.row_bytes <= 0) var.row_bytes = g_var_rb.load();
     if (var.bn <= 0) var.bn = g_var_bn.load();
@@ -3020,7 +3025,7 @@ static int launch_stage(const b200d2_view& v, const b200d2_batch& b, const TcGeo
                                               U->nntile[2], U->nperm)));
         break;
       }
-      if (P <= kNormvMaxP) {
+      if (P <= kNormvMaxP && !g.served) {
         const dim3 grid((g.O + 7) / 8);
         switch (P) {
           case 1: tc_normv_kernel<1><<<grid, 256, 0, s>>>(wcomp, g.Kq, q, g.O, normx, na, na_hl, cc); break;
@@ -3314,13 +3319,14 @@ unsigned long long launch_counter();
 void uncount_launch(unsigned n);
 
 int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws, size_t ws_bytes,
-           cudaStream_t s, const int* d_proj_need, float* d_eul_cache) {
+           cudaStream_t s, const int* d_proj_need, float* d_eul_cache, bool served) {
   NvtxRange range("b200d2_diff2_coarse_batch");
   int st = check_tc(v, b);
   if (st != B200D2_OK) return st;
   TcGeom g = make_geom(v, b, precision);
   g.d_proj_need = d_proj_need;
   g.d_eul_cache = d_eul_cache;
+  g.served = served;
   if (d_proj_need) g.fused = 0;  // projections may be kept from the last call: separate stages
   if (ws_bytes < g.total) return B200D2_ERR_INVALID;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -3331,6 +3337,7 @@ int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws,
   std::vector<uint64_t> key = batch_key(v, b, precision, ws, ws_bytes, s, dev);
   key.push_back((uint64_t)(uintptr_t)d_proj_need);
   key.push_back((uint64_t)(uintptr_t)d_eul_cache);
+  key.push_back((uint64_t)served);
   std::unique_lock<std::mutex> lk(g_graph_mu);
   BatchGraph* e = nullptr;
   for (BatchGraph& x : g_graphs)
@@ -4066,19 +4073,19 @@ MergedBatch* merged_create(const b200d2_view& v, int N_img, int precision, const
   b.img_stride = N_img;
   m->g = make_geom(v, b, precision, Mrows, false);
   m->g.fused = 0;  // block-diagonal: only the blocks some particle needs
+  m->g.served = 1;
   // CTA pairs while their tiles give every pair of SMs one, else 128-wide
-  // single-CTA tiles (twice the tiles), with k-splits where those are few
+  // single-CTA tiles (twice the tiles)
   if ((long long)m->tiles[2].size() >= num_sms() / 2) {
     m->var.row_bytes = 128;
     m->var.bn = 256;
     m->var.pair = 1;
-    m->var.split = 1;
   } else {
     m->var.row_bytes = 128;
     m->var.bn = 128;
     m->var.pair = 2;
-    m->var.split = 0;
   }
+  m->var.split = 1;
   size_t o = align_up(m->g.total, 256);
   m->off_tab = o;
   auto take = [&](size_t bytes) {
