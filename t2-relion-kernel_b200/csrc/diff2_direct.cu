@@ -8,14 +8,23 @@ int launch_direct_f64(const DirectArgs& a, int P, cudaStream_t s);  // diff2_dir
 
 template <bool CC>
 static int launch_f32(const DirectArgs& a, int P, int K, cudaStream_t s) {
-  switch (dir_rows(a.T)) {
-    case 1: return dir_launch_tt<PairF, 16, 1, CC>(a, P, K, s);
-    case 2: return dir_launch_tt<PairF, 16, 2, CC>(a, P, K, s);
-    case 3: return dir_launch_tt<PairF, 16, 3, CC>(a, P, K, s);
-    case 4: return dir_launch_tt<PairF, 32, 2, CC>(a, P, K, s);
-    case 5: return dir_launch_tt<PairF, 16, 5, CC>(a, P, K, s);
-    case 6: return dir_launch_tt<PairF, 32, 3, CC>(a, P, K, s);
-    default: return dir_launch_tt<PairF, 32, 4, CC>(a, P, K, s);
+  const int rows = dir_rows(a.T);
+  // up to 32 translations the fetches weigh most: two CTAs of 256 threads a SM
+  // hide each other's barriers, unless the tiles are too few to give half of the
+  // SMs a 128-orientation one, where the larger CTAs' clusters spread them better
+  // (image 64, two translations' heights: 64 particles x 4608 orientations 4.07
+  // and 3.77 ms, 64 x 400 0.52 and 0.41; 8 x 400 80 and 103 us, 1 x 4608 96 and
+  // 104 us; 49 translations: 8 x 1703 at image 96 0.74 and 1.03 ms)
+  if (rows <= 2 && 2LL * P * ((a.O + 127) / 128) >= dir_sms())
+    return rows == 1 ? dir_launch_tt<PairF, 256, 16, 1, CC>(a, P, K, s) : dir_launch_tt<PairF, 256, 16, 2, CC>(a, P, K, s);
+  switch (rows) {
+    case 1: return dir_launch_tt<PairF, 512, 16, 1, CC>(a, P, K, s);
+    case 2: return dir_launch_tt<PairF, 512, 16, 2, CC>(a, P, K, s);
+    case 3: return dir_launch_tt<PairF, 512, 16, 3, CC>(a, P, K, s);
+    case 4: return dir_launch_tt<PairF, 512, 32, 2, CC>(a, P, K, s);
+    case 5: return dir_launch_tt<PairF, 512, 16, 5, CC>(a, P, K, s);
+    case 6: return dir_launch_tt<PairF, 512, 32, 3, CC>(a, P, K, s);
+    default: return dir_launch_tt<PairF, 512, 32, 4, CC>(a, P, K, s);
   }
 }
 
@@ -28,13 +37,15 @@ int minloc_preload();  // minloc.cu
 
 // Every kernel a FP32 request can launch.
 int direct_preload() {
-  cudaError_t e = dir_preload_tt<PairF, 16, 1, false>();
-  if (e == cudaSuccess) e = dir_preload_tt<PairF, 16, 2, false>();
-  if (e == cudaSuccess) e = dir_preload_tt<PairF, 16, 3, false>();
-  if (e == cudaSuccess) e = dir_preload_tt<PairF, 32, 2, false>();
-  if (e == cudaSuccess) e = dir_preload_tt<PairF, 16, 5, false>();
-  if (e == cudaSuccess) e = dir_preload_tt<PairF, 32, 3, false>();
-  if (e == cudaSuccess) e = dir_preload_tt<PairF, 32, 4, false>();
+  cudaError_t e = dir_preload_tt<PairF, 256, 16, 1, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 256, 16, 2, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 512, 16, 1, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 512, 16, 2, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 512, 16, 3, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 512, 32, 2, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 512, 16, 5, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 512, 32, 3, false>();
+  if (e == cudaSuccess) e = dir_preload_tt<PairF, 512, 32, 4, false>();
   return e == cudaSuccess ? minloc_preload() : status_from_cuda(e);
 }
 

@@ -6,10 +6,10 @@ namespace b200d2 {
 template <bool CC>
 static int launch_f64(const DirectArgs& a, int P, int K, cudaStream_t s) {
   const int tt = dir_rows(a.T);
-  if (tt <= 1) return dir_launch_tt<PairD, 16, 1, CC>(a, P, K, s);
-  if (tt <= 2) return dir_launch_tt<PairD, 16, 2, CC>(a, P, K, s);
-  if (tt <= 4) return dir_launch_tt<PairD, 16, 4, CC>(a, P, K, s);
-  return dir_launch_tt<PairD, 16, 8, CC>(a, P, K, s);
+  if (tt <= 1) return dir_launch_tt<PairD, 512, 16, 1, CC>(a, P, K, s);
+  if (tt <= 2) return dir_launch_tt<PairD, 512, 16, 2, CC>(a, P, K, s);
+  if (tt <= 4) return dir_launch_tt<PairD, 512, 16, 4, CC>(a, P, K, s);
+  return dir_launch_tt<PairD, 512, 16, 8, CC>(a, P, K, s);
 }
 
 int launch_direct_f64(const DirectArgs& a, int P, cudaStream_t s) {

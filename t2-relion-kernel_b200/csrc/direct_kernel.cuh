@@ -8,37 +8,45 @@
 // (translatePixel), the squared differences summed in the working precision.
 //
 // B200 design (not the reference's loop structure):
-//  * a CTA of 512 threads owns an output tile of one particle, 16 to 128
-//    translations by 32, 64 or 128 orientations; a cluster of 1, 2, 4 or 8 CTAs shares a tile
-//    and splits its pixels, so that few tiles still reach every SM.  The
-//    cluster's partial sums are added through distributed shared memory in
-//    rank order, so each output is written once and the result does not depend
-//    on timing;
+//  * a CTA of 512 threads (256 and two CTAs a SM where up to 32 translations
+//    leave the fetches the most work) owns an output tile of one particle, 16
+//    to 128 translations by 16 to 128 orientations; a cluster of 1, 2, 4 or 8
+//    CTAs shares a tile and splits its pixels, so that few tiles still reach
+//    every SM.  The cluster's partial sums are added through distributed shared
+//    memory in rank order, so each output is written once and the result does
+//    not depend on timing;
 //  * the pixels an orientation can see (a prefix of every image row) are
 //    walked in chunks of KC; the others contribute |S|^2 corr/2 = |X|^2 corr/2
 //    to every (o, t), added once per tile;
 //  * per chunk the CTA stages the shifted image S[k][t] and the projections
-//    A[k][o] in shared memory, both scaled by sqrt(corr/2), so that a (o, t,
-//    pixel) costs one subtraction and one multiply-add for each of the two
-//    components: in FP32 two packed (f32x2) instructions, 2 lane operations
-//    each, the real and the imaginary squares in separate sums;
+//    A[k][o] in shared memory, neighbouring lanes on neighbouring orientations
+//    (in-plane rotations of one pixel: 11.5 ms for 64 particles x 4608
+//    orientations on the linear projector, 16.2 with lanes along the pixels).
+//    In FP32 both are scaled by sqrt(corr/2), so that a (o, t, pixel) costs one
+//    subtraction and one multiply-add for each of the two components: two
+//    packed (f32x2) instructions, 2 lane operations each, the real and the
+//    imaginary squares in separate sums.  FP64 and negative or infinite
+//    weights subtract first and weight the square;
 //  * the phase e^{i(x tx + y ty)} is the product of two table entries built
 //    once per CTA (FP64 sincos, rounded), where they fit; else a sincos per
 //    (pixel, translation) as the reference does;
 //  * the next chunk's texture fetches and shifted images are produced while
-//    the current one is summed (two buffers, one barrier a chunk).
+//    the current one is summed (two buffers, one barrier a chunk); its pixels
+//    are copied to shared memory a chunk ahead of that.
 // Bound: the FP32 pipe.  4608 x 113 samples of one particle at image 64: 95 us
 // for 4 lane operations per (o, t, pixel) at 128 a clock and SM, 107 with the
-// tile's 128 translations; 185 us here (the sums' and the staging's
+// tile's 128 translations; 191 us here (the sums' and the staging's
 // instructions together fill the issue slots: a packed instruction takes two),
 // 449 us with a 32-orientation
 // tile per CTA, a sincosf per (pixel, translation, tile) and 5 operations.
 //
 // The CC form (cuda_kernel_diff2_CC_coarse, src/diff2.cuh:691-809) runs the
-// same tiles with S scaled by corr and A plain: one packed multiply-add per
-// (o, t, pixel) for sum corr Re(conj(A) S), and sum corr |A|^2 per orientation;
-// the output is -cross / sqrt(norm), written (or added with accumulate).
-// Pixels outside the projector radius have A = 0 and are skipped.
+// same tiles with S scaled by corr and A plain: two multiply-adds per
+// (o, t, pixel) for sum corr Re(conj(A) S); the output is -cross / sqrt(norm),
+// written (or added with accumulate).  Pixels outside the projector radius have
+// A = 0 and are skipped.  sum corr |A|^2 is added up by the threads that stage
+// A: in the tile it was repeated by every translation's lanes and its registers
+// spilled (64 particles x 4608 x 113: 17.5 ms, now 8.4).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -74,7 +82,8 @@ struct DirectArgs {
   int off_tab;  // byte offset of the row index and the tables in dynamic shared memory
 };
 
-constexpr int kDirThreads = 512;
+// CTAs of so many threads that share a SM
+constexpr int dir_min_ctas(int threads) { return 512 / threads; }
 
 // Pairs (re, im) in the working precision.  FP32 uses packed f32x2
 // instructions on 64-bit registers.
@@ -93,6 +102,11 @@ struct PairF {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
   }
+  __device__ static __forceinline__ void load2(const V* p, V& a, V& b) {  // p: 16-byte aligned
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    a = v.x;
+    b = v.y;
+  }
   __device__ static __forceinline__ V mul(V a, V b) {
     V d;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
@@ -103,15 +117,8 @@ struct PairF {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
   }
-  __device__ static __forceinline__ void load2(const V* p, V& a, V& b) {  // p: 16-byte aligned
-    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
-    a = v.x;
-    b = v.y;
-  }
-  __device__ static __forceinline__ float sum(V v) {
-    float x, y;
+  __device__ static __forceinline__ void parts(V v, float& x, float& y) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
-    return x + y;
   }
 };
 struct PairD {
@@ -121,40 +128,63 @@ struct PairD {
   __device__ static __forceinline__ V make(double x, double y) { return make_double2(x, y); }
   __device__ static __forceinline__ V zero() { return make_double2(0.0, 0.0); }
   __device__ static __forceinline__ V add(V a, V b) { return make_double2(a.x + b.x, a.y + b.y); }
-  __device__ static __forceinline__ V mul(V a, V b) { return make_double2(a.x * b.x, a.y * b.y); }
-  __device__ static __forceinline__ V fma(V a, V b, V c) {
-    return make_double2(::fma(a.x, b.x, c.x), ::fma(a.y, b.y, c.y));
-  }
   __device__ static __forceinline__ void load2(const V* p, V& a, V& b) {
     a = p[0];
     b = p[1];
   }
-  __device__ static __forceinline__ double sum(V v) { return v.x + v.y; }
+  __device__ static __forceinline__ void parts(V v, double& x, double& y) {
+    x = v.x;
+    y = v.y;
+  }
 };
-// Accumulators: the pair in FP32, one sum in FP64 (half the registers; its
-// rounding is far below the FP32 projections' anyway).
-template <class PR, bool PACKED = std::is_same<PR, PairF>::value>
-struct Acc;
-template <class PR>
-struct Acc<PR, true> {
-  typename PR::V v;
-  __device__ __forceinline__ void clear() { v = PR::zero(); }
-  __device__ __forceinline__ void mac(typename PR::V a, typename PR::V b) { v = PR::fma(a, b, v); }
-  __device__ __forceinline__ typename PR::E total() const { return PR::sum(v); }
-};
-template <class PR>
-struct Acc<PR, false> {
+__device__ __forceinline__ void copy_async(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The sums of one (orientation, translation) over the pixels.
+//  FP32 diff2: the pair of its squares, with A and S scaled by sqrt(corr/2)
+//    (mac), or the weight in the sum (weighted).
+//  FP64 diff2: the weight is in the sum.
+//  CC: one sum; S carries corr.
+template <class PR, bool CC>
+struct Acc {
   typename PR::E v;
   __device__ __forceinline__ void clear() { v = 0; }
-  __device__ __forceinline__ void mac(typename PR::V a, typename PR::V b) { v = ::fma(a.y, b.y, ::fma(a.x, b.x, v)); }
+  __device__ __forceinline__ void mac(typename PR::V a, typename PR::V b) {  // CC: a, b; diff2: not used
+    typename PR::E ax, ay, bx, by;
+    PR::parts(a, ax, ay);
+    PR::parts(b, bx, by);
+    v = ::fma(ax, bx, ::fma(ay, by, v));
+  }
+  __device__ __forceinline__ void weighted(typename PR::V d, typename PR::E w) {
+    typename PR::E x, y;
+    PR::parts(d, x, y);
+    v = ::fma(::fma(x, x, y * y), w, v);
+  }
   __device__ __forceinline__ typename PR::E total() const { return v; }
+};
+template <>
+struct Acc<PairF, false> {
+  PairF::V v;
+  __device__ __forceinline__ void clear() { v = PairF::zero(); }
+  __device__ __forceinline__ void mac(PairF::V a, PairF::V b) { v = PairF::fma(a, b, v); }
+  __device__ __forceinline__ void weighted(PairF::V d, float w) {
+    v = PairF::fma(PairF::mul(d, PairF::make(w, w)), d, v);
+  }
+  __device__ __forceinline__ float total() const {
+    float x, y;
+    PairF::parts(v, x, y);
+    return x + y;
+  }
 };
 
 // A listed pixel of a chunk, for the shifted images (x and its image row's
-// place among the CTA's rows as offsets into the phase tables; the image value
-// times its scale, sqrt(w), or w for CC, negated for diff2: A - S is an add)
-// and for the projections (coordinates, their scale, and the weight left for
-// the sum: 1, or w where the scale is 1).
+// place among the CTA's rows as offsets into the phase tables; the image value,
+// times sqrt(corr/2) for FP32 diff2, times corr for CC; negated for diff2:
+// A - S is an add) and for the projections (coordinates, their scale, and the
+// weight left for the sum).
 template <class E>
 struct alignas(16) ChunkPixel {
   int xo, yo;
@@ -183,22 +213,22 @@ __device__ __forceinline__ int row_count(const b200d2_view& v, int iy, int N_img
 
 // Shared memory of a tile configuration: the two buffers (or the partial
 // sums), the row index and, where they fit, the phase tables.
-template <class PR, int L, int TT, int TO>
+template <class PR, int NT, int L, int TT, int TO>
 struct DirCfg {
-  static constexpr int BT = L * TT, BO = kDirThreads / L * TO;
+  static constexpr int BT = L * TT, BO = NT / L * TO;
   // row stride of the projections: the stores of one orientation's pixels, a
   // half-warp's, shift by 16 bytes a row (8 where a thread reads one at a time)
   static constexpr int LA = BO + (TO > 1 && sizeof(typename PR::V) == 8 ? 2 : 1);
   static constexpr size_t kTiles = 2 * PR::KC * (BT + LA) * sizeof(typename PR::V);
-  static constexpr size_t kPart = ((size_t)BO * BT + BO) * sizeof(typename PR::E);
+  static constexpr size_t kPart = ((size_t)BO * BT + BO + NT) * sizeof(typename PR::E);
   static constexpr size_t kBase = ((kTiles > kPart ? kTiles : kPart) + 15) / 16 * 16;
 };
-template <class PR, int L, int TT, int TO, bool CC>
-__global__ void __launch_bounds__(kDirThreads, 1) diff2_direct_kernel(const __grid_constant__ DirectArgs a) {
+template <class PR, int NT, int L, int TT, int TO, bool CC>
+__global__ void __launch_bounds__(NT, dir_min_ctas(NT)) diff2_direct_kernel(const __grid_constant__ DirectArgs a) {
   using E = typename PR::E;
   using V = typename PR::V;
-  constexpr int BT = L * TT, BO = kDirThreads / L * TO, NT = kDirThreads, KC = PR::KC;
-  constexpr int LA = DirCfg<PR, L, TT, TO>::LA;
+  constexpr int BT = L * TT, BO = NT / L * TO, KC = PR::KC;
+  constexpr int LA = DirCfg<PR, NT, L, TT, TO>::LA;
   constexpr int NF = (BO * KC + NT - 1) / NT;  // projections a thread stages per chunk
   extern __shared__ __align__(16) uint8_t dir_smem[];
   // [2][KC][BT] shifted images, [2][KC][LA] projections; after the loop the
@@ -213,8 +243,8 @@ __global__ void __launch_bounds__(kDirThreads, 1) diff2_direct_kernel(const __gr
   __shared__ ChunkPixel<E> s_px[3][KC];
   __shared__ ChunkSample<E> s_wt[3][KC];
   __shared__ int s_warp[NT / 32];
+  __shared__ int s_slow[3];  // FP32 diff2: the chunk's weights stay in the sum
   __shared__ E s_red[NT / 32];
-  __shared__ int s_slow[3];  // the chunk has a weight that is negative or not finite
 
   cg::cluster_group cl = cg::this_cluster();
   const int CS = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -331,35 +361,30 @@ __global__ void __launch_bounds__(kDirThreads, 1) diff2_direct_kernel(const __gr
   // a thread's sums: translations t_of(i) and orientations oq TO + j
   const int tq = lane % L, oq = tid / L;
   auto t_of = [&](int i) { return i < (TT & ~1) ? L * (i & ~1) + 2 * tq + (i & 1) : L * (TT - 1) + tq; };
-  Acc<PR> acc[TT][TO], nrm[TO];
-#pragma unroll
-  for (int i = 0; i < TT; ++i)
-#pragma unroll
-    for (int j = 0; j < TO; ++j) acc[i][j].clear();
-#pragma unroll
-  for (int j = 0; j < TO; ++j) nrm[j].clear();
+  Acc<PR, CC> acc[TT][TO];
 
   const int nchunk = (ke - kb + KC - 1) / KC;
-  // Pixels of a chunk into slot c % 3, by the first lanes of warp c % 16: their
-  // places and loads first, the values when they are stored.
-  struct {
-    int x, y, row;
+  // FP32 diff2 scales A and S by sqrt(corr/2) before it subtracts them
+  constexpr bool kScaled = !CC && std::is_same<E, float>::value;
+  // Pixels of a chunk into slot c % 3, by the first lanes of warp c % (NT / 32):
+  // their places and loads first (into shared memory: registers are short here),
+  // the values a chunk later, when they have landed.
+  struct RawPixel {
+    int x, row;
     float re, im, corr;
-    bool zero, there;
-  } np;
+  };
+  __shared__ RawPixel s_raw[4][KC];
   auto begin_pixels = [&](int c) {
     if (warp != c % (NT / 32) || lane >= KC) return;
     const int k = kb + c * KC + lane;
-    np.there = k < ke;
-    if (np.there) {
-      const int iy = row_of(k), i = iy * v.imgX + k - s_row[iy];
-      np.x = k - s_row[iy];
-      np.y = iy > v.maxR ? iy - v.imgY : iy;
-      np.row = iy - row0;
-      np.re = g_re[i];
-      np.im = g_im[i];
-      np.corr = g_corr[i];
-      np.zero = filtered(np.x, np.y);
+    if (k < ke) {
+      RawPixel& r = s_raw[c & 3][lane];
+      const int iy = row_of(k), x = k - s_row[iy], i = iy * v.imgX + x;
+      r.x = x;
+      r.row = iy;
+      copy_async(&r.re, g_re + i);
+      copy_async(&r.im, g_im + i);
+      copy_async(&r.corr, g_corr + i);
     }
   };
   auto end_pixels = [&](int c) {
@@ -370,38 +395,42 @@ __global__ void __launch_bounds__(kDirThreads, 1) diff2_direct_kernel(const __gr
       ChunkSample<E> g;
       q.xo = q.yo = 0;
       g.fx = g.fy = 0.f;
-      q.xr = q.xi = g.sa = E(0);  // past the end: zero weight
-      g.wk = CC ? E(0) : E(1);
-      if (np.there) {
-        const E re = np.zero ? E(0) : (E)np.re, im = np.zero ? E(0) : (E)np.im;
-        const float cf = np.corr;
-        q.xo = np.x * BT;
-        q.yo = np.row * BT;
-        g.fx = (float)np.x;
-        g.fy = (float)np.y;
+      q.xr = q.xi = g.sa = g.wk = E(0);  // past the end: the origin, without weight
+      if (kb + c * KC + lane < ke) {
+        copy_async_wait();
+        const RawPixel& r = s_raw[c & 3][lane];
+        const int x = r.x, y = r.row > v.maxR ? r.row - v.imgY : r.row;
+        const bool zero = filtered(x, y);
+        const E re = zero ? E(0) : (E)r.re, im = zero ? E(0) : (E)r.im;
+        const float cf = r.corr;
+        q.xo = x * BT;
+        q.yo = (r.row - row0) * BT;
+        g.fx = (float)x;
+        g.fy = (float)y;
+        g.sa = E(1);
         if (CC) {
-          q.xr = (E)cf * re;
-          q.xi = (E)cf * im;
-          g.sa = E(1);
           g.wk = (E)cf;
-        } else if (cf >= 0.f && cf < __int_as_float(0x7f800000)) {
-          const E sc = sqrt((E)(cf / 2));
-          q.xr = -sc * re;
-          q.xi = -sc * im;
-          g.sa = sc;
-        } else {  // no real square root: the weight stays in the sum
+          q.xr = g.wk * re;
+          q.xi = g.wk * im;
+        } else if (kScaled && cf >= 0.f && cf < __int_as_float(0x7f800000)) {
+          g.sa = sqrt((E)(cf / 2));
+          g.wk = E(1);
+          q.xr = -g.sa * re;
+          q.xi = -g.sa * im;
+        } else {
+          g.wk = (E)(cf / 2);
           q.xr = -re;
           q.xi = -im;
-          g.sa = E(1);
-          g.wk = (E)(cf / 2);
           slow = true;
         }
       }
       s_px[c % 3][lane] = q;
       s_wt[c % 3][lane] = g;
     }
-    slow = __any_sync(0xffffffffu, slow);
-    if (lane == 0) s_slow[c % 3] = slow;
+    if (kScaled) {
+      slow = __any_sync(0xffffffffu, slow);
+      if (lane == 0) s_slow[c % 3] = slow;
+    }
   };
   // shifted images of chunk c
   auto shifted = [&](int c, int k, int t) {
@@ -436,16 +465,21 @@ __global__ void __launch_bounds__(kDirThreads, 1) diff2_direct_kernel(const __gr
     }
   };
   PixelFetch<NF> f;
-  const int ak = tid % KC;  // the pixel whose projections this thread stages, for orientations tid / KC + ...
+  E nrm[NF];  // CC: this thread's share of sum corr |A|^2 of the orientations it stages
+#pragma unroll
+  for (int u = 0; u < NF; ++u) nrm[u] = E(0);
+  // sample u of a thread: pixel a_k(u), orientation a_o(u) of the chunk's tile
+  auto a_k = [&](int u) { return (tid + u * NT) / BO; };
+  auto a_o = [&](int u) { return (tid + u * NT) % BO; };
   auto fetch_A = [&](int c) {
-    const ChunkSample<E> g = s_wt[c % 3][ak];
     float fx[NF], fy[NF];
     const float* e[NF];
 #pragma unroll
     for (int u = 0; u < NF; ++u) {
-      fx[u] = g.fx;
-      fy[u] = g.fy;
-      e[u] = s_eul[min(tid / KC + u * (NT / KC), BO - 1)];
+      const int k = min(a_k(u), KC - 1);
+      fx[u] = s_wt[c % 3][k].fx;
+      fy[u] = s_wt[c % 3][k].fy;
+      e[u] = s_eul[min(a_o(u), BO - 1)];
     }
     f.issue(v, fx, fy, e);
   };
@@ -453,83 +487,90 @@ __global__ void __launch_bounds__(kDirThreads, 1) diff2_direct_kernel(const __gr
     V* d = s_A + (c & 1) * KC * LA;
 #pragma unroll
     for (int u = 0; u < NF; ++u) {
-      const int o = tid / KC + u * (NT / KC);
-      if (BO * KC % NT != 0 && o >= BO) continue;
+      const int k = a_k(u), o = a_o(u);
+      if (BO * KC % NT != 0 && (o >= BO || k >= KC)) continue;
       const float2 b = f.finish(u);
-      const E sc = CC ? E(1) : s_wt[c % 3][ak].sa;
-      d[ak * LA + o] = PR::make(sc * (E)b.x, sc * (E)b.y);
+      E x = (E)b.x, y = (E)b.y;
+      if (CC) nrm[u] = fma(fma(x, x, y * y), s_wt[c % 3][k].wk, nrm[u]);
+      if (kScaled) {
+        x *= s_wt[c % 3][k].sa;
+        y *= s_wt[c % 3][k].sa;
+      }
+      d[k * LA + o] = PR::make(x, y);
     }
   };
-  for (int c = 0; c < 2; ++c) {
-    begin_pixels(c);
-    end_pixels(c);
-  }
-  __syncthreads();  // the tables and the first two chunks' pixels
-  if (nchunk > 0) {
-    fetch_A(0);
-    stage_S(0);
-    store_A(0);
-  }
-  for (int c = 0; c < nchunk; ++c) {
-    __syncthreads();  // chunk c's tiles and chunk c + 1's pixels are there; chunk c - 1's tiles are free
-    auto stage = [&]() {  // chunk c + 1's tiles and chunk c + 2's pixels
-      begin_pixels(c + 2);
-      if (c + 1 < nchunk) {
-        fetch_A(c + 1);
-        stage_S(c + 1);
-      }
-      end_pixels(c + 2);
-      if (c + 1 < nchunk) store_A(c + 1);
-    };
+  auto sums = [&](int c, auto weighted) {
+    constexpr bool W = decltype(weighted)::value;
     const V* S = s_S + (c & 1) * KC * BT;
     const V* A = s_A + (c & 1) * KC * LA;
-    auto sums = [&](auto weighted) {
-      constexpr bool W = decltype(weighted)::value;
-#pragma unroll (W ? 1 : KC)
-      for (int k = 0; k < KC; ++k) {
-        V sv[TT], av[TO];
+#pragma unroll (W && kScaled ? 1 : KC)
+    for (int k = 0; k < KC; ++k) {
+      V sv[TT], av[TO];
 #pragma unroll
-        for (int i = 0; i + 1 < TT; i += 2) PR::load2(S + k * BT + L * i + 2 * tq, sv[i], sv[i + 1]);
-        if (TT & 1) sv[TT - 1] = S[k * BT + L * (TT - 1) + tq];
-        if constexpr (TO == 1) {
-          av[0] = A[k * LA + oq];
-        } else {
+      for (int i = 0; i + 1 < TT; i += 2) PR::load2(S + k * BT + L * i + 2 * tq, sv[i], sv[i + 1]);
+      if (TT & 1) sv[TT - 1] = S[k * BT + L * (TT - 1) + tq];
+      if constexpr (TO == 1) {
+        av[0] = A[k * LA + oq];
+      } else {
 #pragma unroll
-          for (int j = 0; j < TO; j += 2) PR::load2(A + k * LA + oq * TO + j, av[j], av[j + 1]);
-        }
-        if (CC) {
-          const V w = PR::make(s_wt[c % 3][k].wk, s_wt[c % 3][k].wk);
-#pragma unroll
-          for (int j = 0; j < TO; ++j) nrm[j].mac(PR::mul(av[j], w), av[j]);
-#pragma unroll
-          for (int i = 0; i < TT; ++i)
-#pragma unroll
-            for (int j = 0; j < TO; ++j) acc[i][j].mac(av[j], sv[i]);
-        } else {
-          const V w = W ? PR::make(s_wt[c % 3][k].wk, s_wt[c % 3][k].wk) : PR::zero();
-#pragma unroll
-          for (int i = 0; i < TT; ++i)
-#pragma unroll
-            for (int j = 0; j < TO; ++j) {
-              const V d = PR::add(av[j], sv[i]);
-              acc[i][j].mac(W ? PR::mul(d, w) : d, d);
-            }
-        }
+        for (int j = 0; j < TO; j += 2) PR::load2(A + k * LA + oq * TO + j, av[j], av[j + 1]);
       }
-    };
-    // two warps of each sub-partition stage first and two sum first, so that
-    // the staging's loads and integer work run beside the FP32 pipe's sums
-    const int turn = (warp >> 2) & 1;
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      if (h == turn)
-        stage();
-      else if (!CC && s_slow[c % 3])
-        sums(std::true_type());
-      else
-        sums(std::false_type());
+      [[maybe_unused]] const E w = W ? s_wt[c % 3][k].wk : E(0);
+#pragma unroll
+      for (int i = 0; i < TT; ++i)
+#pragma unroll
+        for (int j = 0; j < TO; ++j) {
+          if constexpr (CC) {
+            acc[i][j].mac(av[j], sv[i]);
+          } else {
+            const V d = PR::add(av[j], sv[i]);
+            if constexpr (W)
+              acc[i][j].weighted(d, w);
+            else
+              acc[i][j].mac(d, d);
+          }
+        }
     }
-  }
+  };
+  auto walk = [&]() {  // the sums over this CTA's pixels
+#pragma unroll
+    for (int i = 0; i < TT; ++i)
+#pragma unroll
+      for (int j = 0; j < TO; ++j) acc[i][j].clear();
+    for (int c = 0; c < 3; ++c) begin_pixels(c);
+    for (int c = 0; c < 2; ++c) end_pixels(c);
+    __syncthreads();  // the tables and the first two chunks' pixels
+    if (nchunk > 0) {
+      fetch_A(0);
+      stage_S(0);
+      store_A(0);
+    }
+    for (int c = 0; c < nchunk; ++c) {
+      __syncthreads();  // chunk c's tiles and chunk c + 1's pixels are there; chunk c - 1's tiles are free
+      auto stage = [&]() {  // chunk c + 1's tiles and chunk c + 2's pixels
+        begin_pixels(c + 3);
+        if (c + 1 < nchunk) {
+          fetch_A(c + 1);
+          stage_S(c + 1);
+        }
+        end_pixels(c + 2);
+        if (c + 1 < nchunk) store_A(c + 1);
+      };
+      // two warps of each sub-partition stage first and two sum first, so that
+      // the staging's loads and integer work run beside the FP32 pipe's sums
+      const int turn = (warp >> 2) & 1;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        if (h == turn)
+          stage();
+        else if (!CC && (!kScaled || s_slow[c % 3]))
+          sums(c, std::true_type());
+        else if (CC || kScaled)
+          sums(c, std::false_type());
+      }
+    }
+  };
+  walk();
 
   // the out-of-radius constant of this CTA
 #pragma unroll
@@ -551,25 +592,40 @@ __global__ void __launch_bounds__(kDirThreads, 1) diff2_direct_kernel(const __gr
       *dst = *dst + sum;
     }
   };
+  // partial sums [BO][BT] (clusters) and norms (CC) into this CTA's shared
+  // memory; each rank then adds its share of the tile over the cluster, in rank
+  // order
+  E* part = reinterpret_cast<E*>(dir_smem);
+  E* pnrm = part + BO * BT;
+  if (CC) {
+    // an orientation's pixels were staged by threads BO apart
+    E* pn = pnrm + BO;  // [max(1, NT / BO)][BO]
+    constexpr int G = NT / BO > 1 ? (NT / BO < KC ? NT / BO : KC) : 1;
+    E n = nrm[0];
+#pragma unroll
+    for (int u = 1; u < NF; ++u) n += nrm[u];
+    if (tid < G * BO) pn[tid] = n;
+    __syncthreads();
+    if (tid < BO) {
+      E n = E(0);
+      for (int g = 0; g < G; ++g) n += pn[g * BO + tid];
+      pnrm[tid] = n;
+    }
+  }
   if (CS == 1) {
+    if (CC) __syncthreads();
 #pragma unroll
     for (int j = 0; j < TO; ++j)
 #pragma unroll
       for (int i = 0; i < TT; ++i)
-        put(o0 + oq * TO + j, t0 + t_of(i), CC ? acc[i][j].total() : acc[i][j].total() + out_total, nrm[j].total());
+        put(o0 + oq * TO + j, t0 + t_of(i), CC ? acc[i][j].total() : acc[i][j].total() + out_total, CC ? pnrm[oq * TO + j] : E(0));
     return;
   }
-  // partial sums [BO][BT] and norms into this CTA's shared memory; each rank
-  // then adds its share of the tile over the cluster, in rank order
-  E* part = reinterpret_cast<E*>(dir_smem);
-  E* pnrm = part + BO * BT;
 #pragma unroll
-  for (int j = 0; j < TO; ++j) {
+  for (int j = 0; j < TO; ++j)
 #pragma unroll
     for (int i = 0; i < TT; ++i)
       part[(oq * TO + j) * BT + t_of(i)] = CC ? acc[i][j].total() : acc[i][j].total() + out_total;
-    if (CC && tq == 0) pnrm[oq * TO + j] = nrm[j].total();
-  }
   cl.sync();
   const int e0 = (int)((long long)BO * BT * rank / CS), e1 = (int)((long long)BO * BT * (rank + 1) / CS);
   for (int e = e0 + tid; e < e1; e += NT) {
@@ -587,9 +643,9 @@ constexpr size_t kDirSmem = 212 * 1024;  // dynamic shared memory of a CTA, at m
 
 // Fills the fields that depend on the tile and the shared-memory size; false
 // when the tile does not fit beside the row index of a very tall image.
-template <class PR, int L, int TT, int TO>
+template <class PR, int NT, int L, int TT, int TO>
 static bool dir_smem_layout(DirectArgs& a, size_t& bytes) {
-  using C = DirCfg<PR, L, TT, TO>;
+  using C = DirCfg<PR, NT, L, TT, TO>;
   a.o_tiles = (a.O + C::BO - 1) / C::BO;
   a.off_tab = (int)C::kBase;
   bytes = C::kBase + ((size_t)a.view.imgY + 4) / 4 * 16;
@@ -606,10 +662,10 @@ static bool dir_smem_layout(DirectArgs& a, size_t& bytes) {
   return true;
 }
 
-template <class PR, int L, int TT, int TO, bool CC>
+template <class PR, int NT, int L, int TT, int TO, bool CC>
 static cudaLaunchConfig_t dir_config(cudaLaunchAttribute* at, size_t bytes, int cs) {
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kDirThreads);
+  cfg.blockDim = dim3(NT);
   cfg.dynamicSmemBytes = bytes;
   at->id = cudaLaunchAttributeClusterDimension;
   at->val.clusterDim.x = (unsigned)cs;
@@ -622,20 +678,27 @@ static cudaLaunchConfig_t dir_config(cudaLaunchAttribute* at, size_t bytes, int 
 // Clusters of cs CTAs that run at once (1 CTA per SM: the shared memory and
 // registers of a tile leave no room for two); asked of the runtime once per
 // cluster size, because a GPC's SM count need not be a multiple of it.
-template <class PR, int L, int TT, int TO, bool CC>
+template <class PR, int NT, int L, int TT, int TO, bool CC>
 static int dir_capacity(size_t bytes, int log2_cs) {
   static std::atomic<int> known[4] = {{0}, {0}, {0}, {0}};
   int n = known[log2_cs].load();
   if (n > 0) return n;
   cudaLaunchAttribute at;
-  cudaLaunchConfig_t cfg = dir_config<PR, L, TT, TO, CC>(&at, bytes, 1 << log2_cs);
+  cudaLaunchConfig_t cfg = dir_config<PR, NT, L, TT, TO, CC>(&at, bytes, 1 << log2_cs);
   cfg.gridDim = dim3(1u << log2_cs);
-  if (cudaOccupancyMaxActiveClusters(&n, diff2_direct_kernel<PR, L, TT, TO, CC>, &cfg) != cudaSuccess || n <= 0) {
+  if (cudaOccupancyMaxActiveClusters(&n, diff2_direct_kernel<PR, NT, L, TT, TO, CC>, &cfg) != cudaSuccess || n <= 0) {
     cudaGetLastError();
     n = 1;
   }
   known[log2_cs].store(n);
   return n;
+}
+
+static inline int dir_sms() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
 }
 
 // A tile width and cluster size with its estimated time in lane operations
@@ -651,46 +714,48 @@ struct DirChoice {
 // tables (FP64 sincos) and a fixed part of about 5 us; times the waves of
 // clusters.  One particle at C2 takes 64-orientation tiles on pairs (72 tiles,
 // one wave); 128-wide tiles on clusters of 4 would need 36 clusters at once.
-template <class PR, int L, int TT, int TO, bool CC>
+template <class PR, int NT, int L, int TT, int TO, bool CC>
 static void dir_consider(const DirectArgs& a0, int P, int K, DirChoice& best) {
-  using C = DirCfg<PR, L, TT, TO>;
+  using C = DirCfg<PR, NT, L, TT, TO>;
   constexpr bool D = std::is_same<PR, PairD>::value;
   DirectArgs a = a0;
   size_t bytes = 0;
-  if (!dir_smem_layout<PR, L, TT, TO>(a, bytes)) return;
+  if (!dir_smem_layout<PR, NT, L, TT, TO>(a, bytes)) return;
   static std::atomic<unsigned long long> opted{0};
-  if (smem_opt_in(diff2_direct_kernel<PR, L, TT, TO, CC>, (int)kDirSmem, opted) != cudaSuccess) {
+  if (smem_opt_in(diff2_direct_kernel<PR, NT, L, TT, TO, CC>, (int)kDirSmem, opted) != cudaSuccess) {
     cudaGetLastError();
     return;
   }
+  const int sms = dir_sms();
   const double tiles = (double)P * a.o_tiles * ((a.T + C::BT - 1) / C::BT);
   // lane operations a sample, or what its shared-memory reads take
   const double lds = 128.0 * (D ? 2.0 : 1.0) * (2.0 * TT + TO) / (32.0 * TT * TO);
   const double ops = std::max((CC ? 2.0 : 4.0) * (D ? 2 : 1), lds);
   for (int l = 0; l < 4; ++l) {
     const int cs = 1 << l;
-    const double waves = std::ceil(tiles / dir_capacity<PR, L, TT, TO, CC>(bytes, l));
+    const double waves = std::ceil(tiles / dir_capacity<PR, NT, L, TT, TO, CC>(bytes, l));
+    const double loads = std::max(waves, std::ceil(tiles * cs / sms));  // CTAs that the fullest SM works through
     const double share = std::ceil((double)K / cs);
     const double stage = (a.exw ? 18.0 * (D ? 2 : 1) : D ? 300.0 : 60.0) * C::BT + 60.0 * C::BO;
     const double tab = a.exw ? 140.0 * (a.exw + (double)a.view.imgY / cs) * C::BT : 0.0;
-    const double cost = waves * (share * (ops * C::BT * C::BO + stage) + tab + 1.2e6 + (cs > 1 ? 2e5 : 0.0));
+    const double cost = loads * (share * (ops * C::BT * C::BO + stage) + tab) + waves * (1.2e6 + (cs > 1 ? 2e5 : 0.0));
     if (cost < best.cost) best = DirChoice{cost, TO, cs};
   }
 }
 
-template <class PR, int L, int TT, int TO, bool CC>
+template <class PR, int NT, int L, int TT, int TO, bool CC>
 static int dir_launch(const DirectArgs& a0, int P, int cs, cudaStream_t s) {
-  using C = DirCfg<PR, L, TT, TO>;
+  using C = DirCfg<PR, NT, L, TT, TO>;
   DirectArgs a = a0;
   size_t bytes = 0;
-  if (!dir_smem_layout<PR, L, TT, TO>(a, bytes)) return B200D2_ERR_UNSUPPORTED;
+  if (!dir_smem_layout<PR, NT, L, TT, TO>(a, bytes)) return B200D2_ERR_UNSUPPORTED;
   const long long nx = (long long)a.o_tiles * ((a.T + C::BT - 1) / C::BT) * cs;
   if (nx > 0x7fffffffLL || P > 65535) return B200D2_ERR_UNSUPPORTED;
   cudaLaunchAttribute at;
-  cudaLaunchConfig_t cfg = dir_config<PR, L, TT, TO, CC>(&at, bytes, cs);
+  cudaLaunchConfig_t cfg = dir_config<PR, NT, L, TT, TO, CC>(&at, bytes, cs);
   cfg.gridDim = dim3((unsigned)nx, 1, (unsigned)P);
   cfg.stream = s;
-  B200D2_CUDA_TRY(cudaLaunchKernelEx(&cfg, diff2_direct_kernel<PR, L, TT, TO, CC>, a));
+  B200D2_CUDA_TRY(cudaLaunchKernelEx(&cfg, diff2_direct_kernel<PR, NT, L, TT, TO, CC>, a));
   count_launch();
   return status_from_cuda(cudaGetLastError());
 }
@@ -702,30 +767,30 @@ static int dir_launch(const DirectArgs& a0, int P, int cs, cudaStream_t s) {
 // multiples of 32 put 32 lanes along the translations and more orientations in
 // a thread (4 x 4 needs 12 clocks for 16, where 8 x 2 on 16 lanes needs 18: at
 // C2 one particle took 255 us with that).
-template <class PR, int L, int TT, bool CC>
+template <class PR, int NT, int L, int TT, bool CC>
 static int dir_launch_tt(const DirectArgs& a, int P, int K, cudaStream_t s) {
   constexpr int W = L / 16;
   DirChoice c;
-  dir_consider<PR, L, TT, 4 * W, CC>(a, P, K, c);
-  dir_consider<PR, L, TT, 2 * W, CC>(a, P, K, c);
-  dir_consider<PR, L, TT, W, CC>(a, P, K, c);
+  dir_consider<PR, NT, L, TT, 4 * W, CC>(a, P, K, c);
+  dir_consider<PR, NT, L, TT, 2 * W, CC>(a, P, K, c);
+  dir_consider<PR, NT, L, TT, W, CC>(a, P, K, c);
   switch (c.to) {
-    case 4 * W: return dir_launch<PR, L, TT, 4 * W, CC>(a, P, c.cs, s);
-    case 2 * W: return dir_launch<PR, L, TT, 2 * W, CC>(a, P, c.cs, s);
-    case W: return dir_launch<PR, L, TT, W, CC>(a, P, c.cs, s);
+    case 4 * W: return dir_launch<PR, NT, L, TT, 4 * W, CC>(a, P, c.cs, s);
+    case 2 * W: return dir_launch<PR, NT, L, TT, 2 * W, CC>(a, P, c.cs, s);
+    case W: return dir_launch<PR, NT, L, TT, W, CC>(a, P, c.cs, s);
     default: return B200D2_ERR_UNSUPPORTED;
   }
 }
 
 // Loads the tile's kernels (instead of at their first launch, which can wait
 // for running work).
-template <class PR, int L, int TT, bool CC>
+template <class PR, int NT, int L, int TT, bool CC>
 static cudaError_t dir_preload_tt() {
   constexpr int W = L / 16;
   cudaFuncAttributes a;
-  cudaError_t e = cudaFuncGetAttributes(&a, (const void*)diff2_direct_kernel<PR, L, TT, 4 * W, CC>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, (const void*)diff2_direct_kernel<PR, L, TT, 2 * W, CC>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, (const void*)diff2_direct_kernel<PR, L, TT, W, CC>);
+  cudaError_t e = cudaFuncGetAttributes(&a, (const void*)diff2_direct_kernel<PR, NT, L, TT, 4 * W, CC>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, (const void*)diff2_direct_kernel<PR, NT, L, TT, 2 * W, CC>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, (const void*)diff2_direct_kernel<PR, NT, L, TT, W, CC>);
   return e;
 }
 
