@@ -364,8 +364,12 @@ __global__ void __launch_bounds__(NT, dir_min_ctas(NT)) diff2_direct_kernel(cons
   Acc<PR, CC> acc[TT][TO];
 
   const int nchunk = (ke - kb + KC - 1) / KC;
-  // FP32 diff2 scales A and S by sqrt(corr/2) before it subtracts them
+  // FP32 diff2 scales A and S by sqrt(corr/2) before it subtracts them; `plain`
+  // takes the differences first and leaves the weights to the sums
   constexpr bool kScaled = !CC && std::is_same<E, float>::value;
+  bool plain = false;
+  __shared__ float s_x2[2][KC];  // sum corr/2 |X|^2 of the scaled pixels (even and odd chunks)
+  if (kScaled && tid < 2 * KC) s_x2[tid / KC][tid % KC] = 0.f;
   // Pixels of a chunk into slot c % 3, by the first lanes of warp c % (NT / 32):
   // their places and loads first (into shared memory: registers are short here),
   // the values a chunk later, when they have landed.
@@ -412,11 +416,12 @@ __global__ void __launch_bounds__(NT, dir_min_ctas(NT)) diff2_direct_kernel(cons
           g.wk = (E)cf;
           q.xr = g.wk * re;
           q.xi = g.wk * im;
-        } else if (kScaled && cf >= 0.f && cf < __int_as_float(0x7f800000)) {
+        } else if (kScaled && !plain && cf >= 0.f && cf < __int_as_float(0x7f800000)) {
           g.sa = sqrt((E)(cf / 2));
           g.wk = E(1);
           q.xr = -g.sa * re;
           q.xi = -g.sa * im;
+          s_x2[c & 1][lane] += (float)(q.xr * q.xr + q.xi * q.xi);
         } else {
           g.wk = (E)(cf / 2);
           q.xr = -re;
@@ -570,7 +575,34 @@ __global__ void __launch_bounds__(NT, dir_min_ctas(NT)) diff2_direct_kernel(cons
       }
     }
   };
-  walk();
+  if constexpr (kScaled) {
+    // Scaled operands are rounded before they are subtracted: a relative error
+    // of up to 2^-22 sqrt(sum corr/2 |X|^2 / score) in a score (over this CTA's
+    // pixels).  Where one is below kNear of that power the tile is summed
+    // again, differences first, as the error could pass 4e-6; noisy images are
+    // not (ratios around 1), a projection of the volume itself is.
+    constexpr float kNear = 1.f / 256.f;
+    static_assert(2 * KC == 32, "one warp's worth of partial sums");
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      plain = pass > 0;
+      walk();
+      __syncthreads();  // s_x2
+      float near = (&s_x2[0][0])[lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) near += __shfl_xor_sync(0xffffffffu, near, o);
+      near *= kNear;
+      bool below = false;
+#pragma unroll
+      for (int i = 0; i < TT; ++i)
+#pragma unroll
+        for (int j = 0; j < TO; ++j)
+          below |= acc[i][j].total() < near && o0 + oq * TO + j < a.O && t0 + t_of(i) < a.T;
+      if (!__syncthreads_or(below && pass == 0)) break;
+    }
+  } else {
+    walk();
+  }
 
   // the out-of-radius constant of this CTA
 #pragma unroll
