@@ -1084,14 +1084,17 @@ __global__ void __launch_bounds__(kPnThreads, 1)
     *s_abort = 1;
     atomicExch(status, (uint32_t)B200D2_ERR_TIMEOUT);
   };
-  // one lane waits, the warp learns the outcome (and is ordered behind it)
+  // one lane waits, the warp learns the outcome; a shuffle orders no memory, so
+  // a barrier of the warp puts the other lanes' accesses behind the wait
   auto wait = [&](uint64_t* bar, uint32_t parity) {
     int ok = 1;
     if (lane == 0) {
       ok = sm100::mbar_wait_bounded(bar, parity, s_abort, wait_ns) ? 1 : 0;
       if (!ok) give_up();
     }
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    return ok != 0;
   };
   if (warp >= kPnMmaWarps) {
     // ------------------------------------------------ projection warps
