@@ -630,12 +630,14 @@ int b200d2_set_projection_cache(int enable);
 /* Test hook for the give-up path of the bounded device-side waits (no
  * counterpart in the reference, whose waits cannot hang: it recomputes instead
  * of spinning, src/translation_matrix_handler.cuh:145-206).  Sets, process
- * wide, the limit in nanoseconds of the single-CTA contraction's pipeline
- * waits (its shared-memory stage ring and accumulator hand-over); 0 restores
- * the default of 4 s.  When a wait runs out the kernel raises an abort flag
+ * wide, the limit in nanoseconds of the pipeline waits of the single-CTA
+ * contraction (its shared-memory stage ring and accumulator hand-over) and of
+ * the projection kernel that takes the norms along (its shared-memory ring); 0
+ * restores the default of 4 s.  When a wait runs out the kernel raises an abort flag
  * that its other roles see, lets its copies and MMAs in flight finish (those
  * drain waits keep the 4 s limit), frees its tensor memory and returns, and
- * b200d2_workspace_status reports B200D2_ERR_TIMEOUT.  The CTA-pair
+ * b200d2_workspace_status reports B200D2_ERR_TIMEOUT.  Tiles that depend on it
+ * are not written (none where the projection gave up).  The CTA-pair
  * contraction keeps the default limit.  Read when a contraction is launched
  * (plans capture it in their graph).  For tests only: a short limit makes
  * correct runs fail. */

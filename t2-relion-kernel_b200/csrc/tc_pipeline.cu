@@ -54,6 +54,15 @@ namespace b200d2 {
 
 constexpr uint64_t kWaitLimitNs = 4000000000ull;  // 4 s: limit of the device-side waits
 
+// Limit of the pipeline waits of the projection and norm kernel and of the
+// single-CTA contraction, set by b200d2_set_wait_limit_ns for tests of the
+// give-up paths (0: kWaitLimitNs).
+static std::atomic<unsigned long long> g_wait_ns{0};
+static unsigned long long wait_limit() {
+  const unsigned long long ns = g_wait_ns.load();
+  return ns ? ns : kWaitLimitNs;
+}
+
 // ------------------------------------------------------------------ geometry
 constexpr int kMaxSplit = 8;  // largest k-split of a contraction tile (the portable cluster size)
 
@@ -1176,13 +1185,17 @@ __global__ void __launch_bounds__(kPnThreads, 1)
       if (sl < nslab) stage_w(sl);
       cp_async_commit();
     }
+    bool whole = true;
     for (int sl = 0; sl < nslab; ++sl) {
       const int st = sl % NST;
       cp_async_wait<NST - 2>();
       __syncwarp();  // this slab's weights landed; every lane is done with slab sl - 1
       if (sl + NST - 1 < nslab) stage_w(sl + NST - 1);
       cp_async_commit();
-      if (!wait(&s_full[st], (uint32_t)(sl / NST) & 1u)) break;
+      if (!wait(&s_full[st], (uint32_t)(sl / NST) & 1u)) {
+        whole = false;  // no norms from part of the pixels
+        break;
+      }
       const double* cq = sq + st * BO * LD;
       const float* cw = sw + (st * kPnMmaWarps + warp) * C::kRows * LD;
       const int kn = min(KC, Kq - sl * KC);  // a multiple of 16
@@ -1225,7 +1238,7 @@ __global__ void __launch_bounds__(kPnThreads, 1)
 #pragma unroll
     for (int i = 0; i < WM; ++i) {
       const int p = p0 + 8 * i + gid;
-      if (p >= P) continue;
+      if (p >= P || !whole) continue;
       const double nx = normx[p];
 #pragma unroll
       for (int j = 0; j < WN; ++j)
@@ -1459,6 +1472,14 @@ __device__ __forceinline__ void split_range(const GemmArgs& g, int nsplit, int s
   kb1 = g.KB * (s + 1) / nsplit;
 }
 
+// Whether a bounded wait of an earlier stage of this run gave up: its operands
+// are then incomplete and nothing is scored.  (Any status but that one is
+// reported and scored.)  The same for every lane of the calling warp.
+__device__ __forceinline__ bool run_gave_up(const GemmArgs& g) {
+  return __any_sync(0xffffffffu,
+                    *reinterpret_cast<volatile const uint32_t*>(g.status) == (uint32_t)B200D2_ERR_TIMEOUT);
+}
+
 __device__ __forceinline__ uint32_t ordered_bits(float f) {
   const uint32_t u = __float_as_uint(f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -1467,10 +1488,6 @@ __device__ __forceinline__ uint32_t ordered_bits(float f) {
 __device__ __forceinline__ float from_ordered(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
-
-// Pipeline-wait limit of the single-CTA contraction, set by
-// b200d2_set_wait_limit_ns for tests of the give-up path (0: kWaitLimitNs).
-static std::atomic<unsigned long long> g_wait_ns{0};
 
 // Epilogue warps of the contraction kernels: two per TMEM lane quadrant, each
 // draining half of the accumulator's columns.
@@ -2069,6 +2086,7 @@ __global__ void __launch_bounds__(GEN ? kGemmThreadsGen : kGemmThreads, 1)
   const int num_tiles = g.L.tiles ? g.L.ntiles : g.Mtiles * g.Ntiles;
   const int num_items = SPLIT ? num_tiles * g.split : num_tiles;  // SPLIT: one item per CTA
   const int nsplit = SPLIT ? g.split : 1;
+  bool dead = false;  // epilogue warps: an earlier stage gave up, nothing is scored
 
   auto raise_abort = [&]() {
     *s_abort = 1;
@@ -2216,6 +2234,7 @@ __global__ void __launch_bounds__(GEN ? kGemmThreadsGen : kGemmThreads, 1)
     const int half = (warp - 2) >> 2;
     const int row = qd * 32 + lane;
     constexpr int kCols = C::kBN / (EPI / 4);  // columns per epilogue warp
+    dead = run_gave_up(g);                     // (read while the first tile is summed)
     int i = 0;
     for (int item = blockIdx.x; item < num_items; item += gridDim.x, ++i) {
       const int b = i & 1;
@@ -2239,7 +2258,7 @@ __global__ void __launch_bounds__(GEN ? kGemmThreadsGen : kGemmThreads, 1)
         const bool fast = !g.L.rows && !g.accumulate && !g.combine64 && o0 + kCols <= g.O;
         float best = __int_as_float(0x7f800000);
         int best_lo = -1;
-        epi_drain<C::kScaled, kCols / 32>(g, x, taddr, o0, vrow, fast, best, best_lo);
+        if (!dead) epi_drain<C::kScaled, kCols / 32>(g, x, taddr, o0, vrow, fast, best, best_lo);
         sm100::tc_fence_before();
         sm100::mbar_arrive(&acce[b]);
         epi_min(g, x, p, vrow, best, best_lo);
@@ -2288,7 +2307,7 @@ __global__ void __launch_bounds__(GEN ? kGemmThreadsGen : kGemmThreads, 1)
       for (int r = 0; r < nsplit; ++r) sm100::st_cluster_u32(sm100::map_to_rank(tmem_slot + 1, (uint32_t)r), 1u);
     __syncthreads();
     sm100::cluster_sync();  // every part and flag has arrived, and nothing remote follows
-    if (epi && !*s_abort) {
+    if (epi && !*s_abort && !dead) {
       float best = __int_as_float(0x7f800000);
       int best_lo = -1;
       if (vrow) {
@@ -2559,6 +2578,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEN ? kGemmThreadsGe
     const int qd = warp & 3;            // TMEM lane quadrant this warp may access
     const int half = (warp - 2) >> 2;  // column half of the 256-wide tile (8 epilogue warps)
     const int row = qd * 32 + lane;
+    const bool dead = run_gave_up(g);  // (read while the first tile is summed)
     int i = 0;
     for (int tile = cl; tile < num_tiles; tile += ncl, ++i) {
       const int b = i & 1;
@@ -2580,8 +2600,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEN ? kGemmThreadsGe
       const bool fast = !g.L.rows && !g.accumulate && !g.combine64 && o0 + kCols <= g.O;
       float best = __int_as_float(0x7f800000);
       int best_lo = -1;
-      epi_drain<C::kScaled, kCols / 32>(g, x, tmem + (uint32_t)(b * 256 + half * kCols) + ((uint32_t)(qd * 32) << 16),
-                                        o0, vrow, fast, best, best_lo);
+      if (!dead)
+        epi_drain<C::kScaled, kCols / 32>(g, x,
+                                          tmem + (uint32_t)(b * 256 + half * kCols) + ((uint32_t)(qd * 32) << 16), o0,
+                                          vrow, fast, best, best_lo);
       sm100::tc_fence_before();
       sm100::mbar_arrive_cluster(acce0 + 8u * (uint32_t)b);  // the even CTA may reuse buffer b
       epi_min(g, x, p, vrow, best, best_lo);
@@ -2788,7 +2810,7 @@ static int launch_gemm_v(const b200d2_batch& b, const TcGeom& g, void* ws, cudaS
   a.inv_sa = ws_at<float>(ws, g.off_sa);
   a.inv_sb = ws_at<float>(ws, g.off_sb);
   a.L = Layout{U ? U->parts : nullptr, U ? U->rows : nullptr, U ? U->tiles[wl] : nullptr, U ? U->ntiles[wl] : 0};
-  a.wait_ns = g_wait_ns.load() ? g_wait_ns.load() : kWaitLimitNs;
+  a.wait_ns = wait_limit();
   set_gen_args(a, g, ws);
   constexpr int kSmem = gemm_smem_bytes<C, GEN>();
   // the shared-memory opt-in is a per-device function attribute
@@ -3005,7 +3027,7 @@ static int launch_stage(const b200d2_view& v, const b200d2_batch& b, const TcGeo
       const int cc = b.score == B200D2_SCORE_CC;
       if constexpr (!kScaled) {
         if (g.fused) {
-          B200D2_CUDA_TRY((launch_project_norm<PREC>(s, v, b.d_eulers, g, ws, xy, cc, kWaitLimitNs)));
+          B200D2_CUDA_TRY((launch_project_norm<PREC>(s, v, b.d_eulers, g, ws, xy, cc, wait_limit())));
           if (g.P == g.fused) break;
           count_launch();  // the other particles' norms follow, from |B|^2
         }
