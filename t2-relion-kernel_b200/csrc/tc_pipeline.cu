@@ -127,25 +127,43 @@ static int count_inside(const b200d2_view& v, int N_img, int* extent) {
   return n;
 }
 
+// Orientations per CTA of the kernel that projects and takes the norms
+// (tc_project_norm_kernel, one CTA a SM): 32 while that gives two thirds of the
+// SMs a CTA (the weights are read once per CTA), else 16, else (up to 64
+// particles) 8, but never narrower tiles than one wave of CTAs holds (8 to 48
+// particles x 1280 orientations at image 48, whole batch: 8 wide 0.95 to 0.97 of
+// the separate kernels' speed, 16 wide 1.06 to 1.08).
+static int project_norm_tile(int P, int O) {
+  const int sms = num_sms(), want = sms * 2 / 3;
+  auto ctas = [&](int bo) { return (O + bo - 1) / bo; };
+  if (ctas(32) >= want || ctas(16) > sms) return 32;
+  return ctas(16) >= want || P > 64 || ctas(8) > sms ? 16 : 8;
+}
+
 // Particles whose norms the projection kernel takes (TcGeom::fused): the
 // first kFusedMaxP, or none.  None for the FP16 forms (they project twice: their
 // scale comes from the whole row) and for the linear projector (16 scattered
 // loads a sample want more warps than the fused kernel has: 45 particles x 1703
-// orientations at image 48 take 82 us fused, 64 and 21 us apart).  Few
-// orientations give the fused kernel few CTAs.  Up to 64 particles it is the
-// faster one all the same (whole batches of 8 to 64 particles, 72 to 2304
-// orientations, images 20 to 64: 0.94 to 1.51 times, 1.07 in the middle); with
-// more, its MMAs are exposed while tc_norma_kernel spreads the particles over
-// the SMs, so it takes at least 0.47 of the SMs in 16-orientation tiles (65 to 256
-// particles at image 64: 1152 orientations 1.01 to 1.05 times, 576 0.88 to 0.92);
-// and up to kNormvMaxP, where the separate norms only stream |B|^2, two thirds
-// (one particle at image 64: 2304 orientations 1.01 times, 1152 0.84).
+// orientations at image 48 take 82 us fused, 64 and 21 us apart).  From 5 to 64
+// particles it is the faster one (whole batches, 300 to 3200 orientations,
+// images 20 to 96: 0.97 to 2.07 times, 1.13 in the middle).  With more, its MMAs
+// are exposed while tc_norma_kernel spreads the particles over the SMs, so it
+// takes at least 0.47 of the SMs in 16-orientation tiles (65 to 256 particles,
+// images 20 to 96: 1152 orientations 0.97 to 1.25 times, 576 0.87 to 1.2).  Up to
+// kNormvMaxP, where the separate norms only stream |B|^2, tiles of 16 or more
+// have to fill six tenths of the SMs in every wave, and nine tenths for one
+// particle (one at image 64: 2304 orientations 1.02, 4608 1.19, 1600 0.84, 2500
+// 0.82, 3200 0.99 times; four: 1600 1.00, 2500 0.92, 3200 1.07).
 constexpr int kFusedMaxP = 256;
 constexpr int kNormvMaxP = 4;
 static int fused_particles(const b200d2_view& v, int prec, int P, int O) {
   if (prec == B200D2_PREC_FP16 || prec == B200D2_PREC_FP16X3 || v.interp != B200D2_INTERP_TEXTURE) return 0;
-  const int ctas = (O + 15) / 16, sms = num_sms();
-  if (P <= kNormvMaxP ? ctas < sms * 2 / 3 : P > 64 && ctas < sms * 15 / 32) return 0;
+  const int sms = num_sms();
+  if (P <= kNormvMaxP) {
+    const int bo = project_norm_tile(P, O), ctas = (O + bo - 1) / bo, room = (ctas + sms - 1) / sms * sms;
+    if (bo < 16 || 10LL * ctas < (P > 1 ? 6LL : 9LL) * room) return 0;
+  }
+  if (P > 64 && (O + 15) / 16 < sms * 15 / 32) return 0;
   return std::min(P, kFusedMaxP);
 }
 
@@ -1074,6 +1092,10 @@ __global__ void __launch_bounds__(kPnThreads, 1)
   volatile uint32_t* s_abort = &s_abort_word;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int o0 = blockIdx.x * BO;
+  if (o0 >= O) {  // padding of B up to its tiles: zero operands, at once
+    for (int e = tid; e < BO * Kq; e += kPnThreads) store_split<PREC>(bhi, blo, (size_t)o0 * Kq + e, 0.f, 0.f);
+    return;
+  }
   const int mma_active = min(kPnMmaWarps, (P + C::kRows - 1) / C::kRows);
   if (tid == 0) {
     s_abort_word = 0;
@@ -1266,13 +1288,10 @@ static cudaError_t launch_project_norm_v(cudaStream_t s, const b200d2_view& v, c
   return cudaSuccess;
 }
 
-// Orientations per CTA: 32 while that gives two thirds of the SMs a CTA (the
-// weights are read once per CTA), else 16, else (up to 64 particles) 8.
 template <int PREC>
 static cudaError_t launch_project_norm(cudaStream_t s, const b200d2_view& v, const float* eulers, const TcGeom& g,
                                        void* ws, const int2* xy, int cc, unsigned long long wait_ns) {
-  const int want = num_sms() * 2 / 3, P = g.fused;
-  const int bo = (g.O + 31) / 32 >= want ? 32 : ((g.O + 15) / 16 >= want || P > 64) ? 16 : 8;
+  const int P = g.fused, bo = project_norm_tile(P, g.O);
   if (P > 128)
     return bo == 32 ? launch_project_norm_v<PREC, 32, 4>(s, v, eulers, g, ws, xy, cc, wait_ns)
                     : launch_project_norm_v<PREC, 16, 4>(s, v, eulers, g, ws, xy, cc, wait_ns);
