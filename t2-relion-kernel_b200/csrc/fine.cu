@@ -214,13 +214,14 @@ __global__ void __launch_bounds__(kFineThreads) diff2_fine_kernel(
 // halving exchanges); of these the fetches are 27 us, phase 2 is 12, the
 // tables 2.  Eight fetches in flight or four CTAs a SM spill: 80 us.
 constexpr int kFineColsMaxThreads = 288;
-// y table of the launch rule below, [-maxR, max(maxR, imgY - maxR - 1)]; the
-// kernel's own has y >= 0 only, and the rule is kept to the images it was drawn for
-__host__ __device__ inline int fine_cols_eyw(int imgY, int maxR) { return maxR + max(maxR, imgY - maxR - 1) + 1; }
 __host__ __device__ inline int fine_cols_rows(int imgY, int maxR) { return max(maxR, imgY - maxR - 1) + 1; }
-constexpr size_t kFineColsSmem = 160 * 1024;  // tables + q, per CTA (launch rule)
+// Tables, q and sums of a CTA, at most: with its fixed part they stay within the
+// 196 KB step of the shared-memory carve-out.  1024 jobs of 16 translations at
+// image 200 (190 KB): 406 us, 629 with the pixels' own phases below; at image 212
+// (214 KB, which leaves the fetches a 28 KB L1) 561 and 713 with the texture, but
+// 3586 and 2718 with the linear projector.
+constexpr size_t kFineColsSmem = 194 * 1024;
 constexpr int kFineColsHalf = 8;              // translations whose sums are in shared memory at a time
-constexpr size_t kFineColsSums = sizeof(float) * kFineColsHalf * kFineColsMaxThreads;  // largest s_c
 
 // Phase 2 of diff2_fine_cols_kernel for the first NC of NT translations: folded
 // rows [f0, f1) of column `col`, whose q lie imgX apart.
@@ -441,20 +442,18 @@ int launch_fine(const b200d2_view* view, const float* d_eulers, const float* d_r
   if (todo_blocks > 0x7fffffffull) return B200D2_ERR_UNSUPPORTED;
   const size_t exw = (size_t)std::max(view->imgX, view->maxR + 1);
   const size_t tab_bytes = sizeof(float2) * kFineMaxTrans * (exw + view->imgY + view->maxR);
-  const size_t cols_bytes =  // tables + q
-      sizeof(float2) * (kFineMaxTrans * (exw + (size_t)fine_cols_eyw(view->imgY, view->maxR)) + image_size);
+  // one thread per (column, row group), about 256 threads, whole warps
+  const int groups = view->imgX <= 0 ? 1 : std::max(1, std::min(view->imgY, std::min((256 + view->imgX / 2) / view->imgX,
+                                                                                      kFineColsMaxThreads / view->imgX)));
+  const size_t threads = ((size_t)view->imgX * groups + 31) / 32 * 32;
+  const size_t cols_bytes =  // tables, q and the threads' sums
+      sizeof(float2) * (kFineMaxTrans * (exw + (size_t)fine_cols_rows(view->imgY, view->maxR)) + image_size) +
+      sizeof(float) * kFineColsHalf * threads;
   if (view->maxR >= 0 && view->imgX > 0 && view->imgY > 0 && cols_bytes <= kFineColsSmem &&
       view->imgX <= kFineColsMaxThreads) {
-    // one thread per (column, row group), about 256 threads, whole warps
-    const int groups = std::max(1, std::min(view->imgY, std::min((256 + view->imgX / 2) / view->imgX,
-                                                                  kFineColsMaxThreads / view->imgX)));
-    const int threads = (view->imgX * groups + 31) / 32 * 32;
     static std::atomic<unsigned long long> opted{0};  // above 48 KB of dynamic shared memory
-    B200D2_CUDA_TRY(smem_opt_in(diff2_fine_cols_kernel<kFineMaxTrans, CC>, (int)(kFineColsSmem + kFineColsSums), opted));
-    const size_t smem =
-        cols_bytes + sizeof(float) * kFineColsHalf * threads - sizeof(float2) * kFineMaxTrans *
-                         (size_t)(fine_cols_eyw(view->imgY, view->maxR) - fine_cols_rows(view->imgY, view->maxR));
-    diff2_fine_cols_kernel<kFineMaxTrans, CC><<<(unsigned)todo_blocks, threads, smem, (cudaStream_t)stream>>>(
+    B200D2_CUDA_TRY(smem_opt_in(diff2_fine_cols_kernel<kFineMaxTrans, CC>, (int)kFineColsSmem, opted));
+    diff2_fine_cols_kernel<kFineMaxTrans, CC><<<(unsigned)todo_blocks, (unsigned)threads, cols_bytes, (cudaStream_t)stream>>>(
         *view, d_eulers, d_real, d_imag, d_trans_x, d_trans_y, d_corr, d_diff2s, (int)image_size, sum_init, groups,
         d_rot_idx, d_trans_idx, d_job_idx, d_job_num);
   } else if (view->maxR >= 0 && view->imgX > 0 && view->imgY > 0 && tab_bytes <= kFineTableBytes) {
