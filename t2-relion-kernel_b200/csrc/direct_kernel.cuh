@@ -56,6 +56,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "cluster_capacity.h"
 #include "common.cuh"
 
 namespace b200d2 {
@@ -707,23 +708,24 @@ static cudaLaunchConfig_t dir_config(cudaLaunchAttribute* at, size_t bytes, int 
   return cfg;
 }
 
-// Clusters of cs CTAs that run at once (1 CTA per SM: the shared memory and
-// registers of a tile leave no room for two); asked of the runtime once per
-// cluster size, because a GPC's SM count need not be a multiple of it.
+// Clusters of cs CTAs that run at once on the current device (512 threads: 1 CTA
+// per SM; 256: 2 while their shared memory fits twice).
 template <class PR, int NT, int L, int TT, int TO, bool CC>
-static int dir_capacity(size_t bytes, int log2_cs) {
-  static std::atomic<int> known[4] = {{0}, {0}, {0}, {0}};
-  int n = known[log2_cs].load();
-  if (n > 0) return n;
-  cudaLaunchAttribute at;
-  cudaLaunchConfig_t cfg = dir_config<PR, NT, L, TT, TO, CC>(&at, bytes, 1 << log2_cs);
-  cfg.gridDim = dim3(1u << log2_cs);
-  if (cudaOccupancyMaxActiveClusters(&n, diff2_direct_kernel<PR, NT, L, TT, TO, CC>, &cfg) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = 1;
-  }
-  known[log2_cs].store(n);
-  return n;
+static int dir_capacity(size_t bytes, int cs) {
+  static ClusterCapacity known[2];
+  int dev = -1;
+  cudaGetDevice(&dev);
+  return known[bytes > kDirSmem / 2].get(dev, cs, [&]() {
+    cudaLaunchAttribute at;
+    cudaLaunchConfig_t cfg = dir_config<PR, NT, L, TT, TO, CC>(&at, bytes, cs);
+    cfg.gridDim = dim3((unsigned)cs);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, diff2_direct_kernel<PR, NT, L, TT, TO, CC>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return n;
+  });
 }
 
 static inline int dir_sms() {
@@ -765,7 +767,7 @@ static void dir_consider(const DirectArgs& a0, int P, int K, DirChoice& best) {
   const double ops = std::max((CC ? 2.0 : 4.0) * (D ? 2 : 1), lds);
   for (int l = 0; l < 4; ++l) {
     const int cs = 1 << l;
-    const double waves = std::ceil(tiles / dir_capacity<PR, NT, L, TT, TO, CC>(bytes, l));
+    const double waves = std::ceil(tiles / dir_capacity<PR, NT, L, TT, TO, CC>(bytes, cs));
     const double loads = std::max(waves, std::ceil(tiles * cs / sms));  // CTAs that the fullest SM works through
     const double share = std::ceil((double)K / cs);
     const double stage = (a.exw ? 18.0 * (D ? 2 : 1) : D ? 300.0 : 60.0) * C::BT + 60.0 * C::BO;

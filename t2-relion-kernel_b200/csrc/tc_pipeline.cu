@@ -47,6 +47,7 @@
 #include <tuple>
 #include <vector>
 
+#include "cluster_capacity.h"
 #include "common.cuh"
 #include "tc_sm100.cuh"
 
@@ -2720,30 +2721,35 @@ static void set_gen_args(GemmArgs& a, const TcGeom& g, void* ws) {
   a.P = g.P;
 }
 
-// Clusters of n CTAs of a split contraction that run at once, asked of the
-// runtime once per size (a GPC's SM count need not be a multiple of n).
-template <int PREC, int ROWB, int BN, bool GEN>
+// Clusters of n CTAs of a split contraction that run at once on the current
+// device.  Asked of the kernel that reads A; the one that generates it has the
+// SM to itself as well, and takes the same splits (the same sums).
+template <int PREC, int ROWB, int BN>
 static int split_capacity(int n) {
   using C = GemmCfg<PREC, ROWB, BN>;
-  static std::atomic<int> known[kMaxSplit + 1];
-  int m = known[n].load();
-  if (m > 0) return m;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = (unsigned)n;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)n);
-  cfg.blockDim = dim3(GEN ? kGemmThreadsGen : kGemmThreads);
-  cfg.dynamicSmemBytes = gemm_smem_bytes<C, GEN>();
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  if (cudaOccupancyMaxActiveClusters(&m, tc_gemm_kernel<PREC, ROWB, BN, GEN, true>, &cfg) != cudaSuccess || m <= 0) {
-    cudaGetLastError();
-    m = 1;
-  }
-  known[n].store(m);
-  return m;
+  static ClusterCapacity known;
+  int dev = -1;
+  cudaGetDevice(&dev);
+  return known.get(dev, n, [&]() {
+    static std::atomic<unsigned long long> opted{0};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)n;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = gemm_smem_bytes<C, false>();
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int m = 0;
+    if (smem_opt_in(tc_gemm_kernel<PREC, ROWB, BN, false, true>, gemm_smem_bytes<C, false>(), opted) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&m, tc_gemm_kernel<PREC, ROWB, BN, false, true>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return m;
+  });
 }
 
 // k-splits of `tiles` tiles of KB k-blocks: the cluster size with the shortest
@@ -2759,14 +2765,14 @@ static int split_capacity(int n) {
 // 18.4, 16.5, 28, 26; 44, 205: 41, 29, 41, 37, 48, 53; 104, 205: 42, 54, 62,
 // 68, 80, 94; 5, 229: 74, 44, 33, 28, 28, 27.5.
 constexpr double kSplitFixed = 17.0, kSplitDrain = 15.0, kSplitSync = 8.0;
-template <int PREC, int ROWB, int BN, bool GEN>
+template <int PREC, int ROWB, int BN>
 static int auto_split(int tiles, int KB) {
   const int sms = num_sms();
   if (tiles >= sms) return 1;
   int best_n = 1;
   double best = kSplitFixed + kSplitDrain + KB * (ROWB / 64.0);
   for (int n = 2; n <= kMaxSplit && KB * ROWB / n >= 128 && tiles * n <= 2 * sms; ++n) {
-    const int cap = std::max(1, split_capacity<PREC, ROWB, BN, GEN>(n) * 7 / 8);
+    const int cap = std::max(1, split_capacity<PREC, ROWB, BN>(n) * 7 / 8);
     const double waves = (tiles + cap - 1) / cap;
     const double t = waves * (kSplitFixed + kSplitSync + (kSplitDrain + KB * (ROWB / 64.0)) / n);
     if (t < best) {
@@ -2835,7 +2841,7 @@ static int launch_gemm_v(const b200d2_batch& b, const TcGeom& g, void* ws, cudaS
   // the shared-memory opt-in is a per-device function attribute
   static std::atomic<unsigned long long> opted{0}, opted_split{0};
   B200D2_CUDA_TRY(smem_opt_in(tc_gemm_kernel<PREC, ROWB, BN, GEN, true>, kSmem, opted_split));
-  a.split = split > 0 ? std::min(split, kMaxSplit) : auto_split<PREC, ROWB, BN, GEN>(tiles, a.KB);
+  a.split = split > 0 ? std::min(split, kMaxSplit) : auto_split<PREC, ROWB, BN>(tiles, a.KB);
   a.split = std::max(1, std::min(a.split, a.KB));
   if (a.split > 1) {
     if ((long long)tiles * a.split > 0x7fffffffLL) return B200D2_ERR_UNSUPPORTED;
