@@ -208,8 +208,9 @@ extern "C" int b200d2_coarse_weights(const float* d_diff2, int P, int O, int T, 
     if (st != B200D2_OK) return st;
     use_min = mn;
   } else if ((d_min < d_sum + P && d_sum < d_min + P) ||
-             (d_weights && d_min < d_weights + P * n && d_weights < d_min + P)) {
-    // the caller's minima share memory with an output: keep a copy of them
+             (d_weights && d_min < d_weights + P * n && d_weights < d_min + P) ||
+             (reinterpret_cast<const uint8_t*>(d_min) < ws + need && ws < reinterpret_cast<const uint8_t*>(d_min + P))) {
+    // the caller's minima share memory with an output or the workspace: keep a copy of them
     B200D2_CUDA_TRY(cudaMemcpyAsync(mn, d_min, sizeof(double) * P, cudaMemcpyDeviceToDevice, s));
     use_min = mn;
   }
