@@ -3365,7 +3365,7 @@ static cudaStream_t capture_stream(int dev) {
   return cs;
 }
 
-unsigned long long launch_counter();
+unsigned long long thread_launches();
 void uncount_launch(unsigned n);
 
 int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws, size_t ws_bytes,
@@ -3420,7 +3420,7 @@ int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws,
       lk.unlock();
       return tc_launch_pipeline(v, b, precision, g, ws, s);
     }
-    const unsigned long long l0 = launch_counter();
+    const unsigned long long l0 = thread_launches();
     st = status_from_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
     if (st == B200D2_OK) {
       const int st2 = tc_launch_pipeline(v, b, precision, g, ws, cs);
@@ -3435,7 +3435,7 @@ int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws,
       }
     }
     // the launches were counted while capturing; the graph launch below counts them
-    e->launches = (unsigned)(launch_counter() - l0);
+    e->launches = (unsigned)(thread_launches() - l0);
     uncount_launch(e->launches);
     if (st != B200D2_OK || !e->exec) {  // capture not possible: stay with direct launches
       e->exec = nullptr;
@@ -3955,11 +3955,11 @@ extern "C" int b200d2_plan_create(const b200d2_view* view, const float* d_eulers
   if (st == B200D2_OK && (flags & B200D2_PLAN_GRAPH)) {
     st = status_from_cuda(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
     if (st == B200D2_OK) {
-      const unsigned long long l0 = launch_counter();
+      const unsigned long long l0 = thread_launches();
       const int st2 = plan_pipeline(p, p->stream, p->var);
       const cudaError_t e = cudaStreamEndCapture(p->stream, &p->graph);
       st = st2 != B200D2_OK ? st2 : status_from_cuda(e);
-      p->launches = (unsigned)(launch_counter() - l0);
+      p->launches = (unsigned)(thread_launches() - l0);
       uncount_launch(p->launches);
     }
     if (st == B200D2_OK) st = status_from_cuda(cudaGraphInstantiate(&p->exec, p->graph, 0));
