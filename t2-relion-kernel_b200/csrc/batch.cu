@@ -22,7 +22,7 @@ int minloc(const float* d, long long n, int P, double* mn, long long* arg, cudaS
 size_t tc_workspace_bytes(const b200d2_view& view, const b200d2_batch& b, int precision, bool reserve = true);
 int tc_run(const b200d2_view& view, const b200d2_batch& b, int precision, void* ws,
            size_t ws_bytes, cudaStream_t s, const int* d_proj_need = nullptr,
-           float* d_eul_cache = nullptr, bool served = false);
+           float* d_eul_cache = nullptr, bool served = false, bool separate = false);
 bool tc_projection_layout(const b200d2_view& v, const b200d2_batch& b, int precision, std::vector<uint64_t>& key);
 
 static int validate(const b200d2_view* v, const b200d2_batch* b) {
@@ -155,14 +155,18 @@ int single_particle_tc(const b200d2_view& v, const float* tx, const float* ty, c
   if (st != B200D2_OK) return st;
   const size_t need = tc_workspace_bytes(v, b, precision);
   std::vector<uint64_t> key;
-  const bool cacheable = g_proj_cache.load() != 0 && tc_projection_layout(v, b, precision, key);
+  // projections that could be kept take their norms in the separate kernels
+  // whether or not they are (the norms' sums run in another order in the kernel
+  // that projects, and the scores are to be the same either way)
+  const bool separate = tc_projection_layout(v, b, precision, key);
+  const bool cacheable = g_proj_cache.load() != 0 && separate;
   std::lock_guard<std::mutex> lk(g_owned_mu);
   OwnedWorkspace* w = nullptr;
   st = owned_workspace(s, need, &w);
   if (st != B200D2_OK) return st;
   if (!cacheable) {
     w->key.clear();
-    return tc_run(v, b, precision, w->ptr, need, s);
+    return tc_run(v, b, precision, w->ptr, need, s, nullptr, nullptr, false, separate);
   }
   uint32_t pf;
   memcpy(&pf, &v.padding_factor, 4);

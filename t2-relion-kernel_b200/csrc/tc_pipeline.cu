@@ -3369,7 +3369,7 @@ unsigned long long thread_launches();
 void uncount_launch(unsigned n);
 
 int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws, size_t ws_bytes,
-           cudaStream_t s, const int* d_proj_need, float* d_eul_cache, bool served) {
+           cudaStream_t s, const int* d_proj_need, float* d_eul_cache, bool served, bool separate) {
   NvtxRange range("b200d2_diff2_coarse_batch");
   int st = check_tc(v, b);
   if (st != B200D2_OK) return st;
@@ -3377,7 +3377,7 @@ int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws,
   g.d_proj_need = d_proj_need;
   g.d_eul_cache = d_eul_cache;
   g.served = served;
-  if (d_proj_need) g.fused = 0;  // projections may be kept from the last call: separate stages
+  if (separate || d_proj_need) g.fused = 0;  // projections may be kept from the last call: separate stages
   if (ws_bytes < g.total) return B200D2_ERR_INVALID;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (!g_batch_graphs.load() || cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
@@ -3388,6 +3388,7 @@ int tc_run(const b200d2_view& v, const b200d2_batch& b, int precision, void* ws,
   key.push_back((uint64_t)(uintptr_t)d_proj_need);
   key.push_back((uint64_t)(uintptr_t)d_eul_cache);
   key.push_back((uint64_t)served);
+  key.push_back((uint64_t)separate);
   std::unique_lock<std::mutex> lk(g_graph_mu);
   BatchGraph* e = nullptr;
   for (BatchGraph& x : g_graphs)
