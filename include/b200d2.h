@@ -560,7 +560,8 @@ int b200d2_set_combine(int mode);
  * (b200d2_diff2_coarse_batch, _stage, _static and the server), process-wide:
  * row_bytes 64 or 128 (k-block row width), tile_n 256 or 128 (orientations
  * per tile), split = k-splits per tile (a cluster of up to 8 CTAs, whose
- * partial sums are added in split order in FP64), pair = 1 for CTA-pair tiles
+ * partial sums are added in split order in FP64; fewer where that would pass two
+ * waves of CTAs, none where the tiles fill the GPU), pair = 1 for CTA-pair tiles
  * (a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs;
  * 256-wide, no k-splits), 2 for single-CTA tiles.  0 in any field restores the
  * default (256-wide tiles, CTA pairs when the pair tiles fill the GPU, 128-wide

@@ -2765,6 +2765,13 @@ static int split_capacity(int n) {
 // 18.4, 16.5, 28, 26; 44, 205: 41, 29, 41, 37, 48, 53; 104, 205: 42, 54, 62,
 // 68, 80, 94; 5, 229: 74, 44, 33, 28, 28, 27.5.
 constexpr double kSplitFixed = 17.0, kSplitDrain = 15.0, kSplitSync = 8.0;
+// The k-splits that a set split (b200d2_set_gemm_variant) gives: none where the
+// tiles fill the GPU by themselves, and no more than two waves of CTAs.
+static int usable_split(int split, long long tiles) {
+  if (tiles >= num_sms()) return 1;
+  return (int)std::max(1LL, std::min<long long>(std::min(split, kMaxSplit), 2LL * num_sms() / std::max(1LL, tiles)));
+}
+
 template <int PREC, int ROWB, int BN>
 static int auto_split(int tiles, int KB) {
   const int sms = num_sms();
@@ -2841,7 +2848,7 @@ static int launch_gemm_v(const b200d2_batch& b, const TcGeom& g, void* ws, cudaS
   // the shared-memory opt-in is a per-device function attribute
   static std::atomic<unsigned long long> opted{0}, opted_split{0};
   B200D2_CUDA_TRY(smem_opt_in(tc_gemm_kernel<PREC, ROWB, BN, GEN, true>, kSmem, opted_split));
-  a.split = split > 0 ? std::min(split, kMaxSplit) : auto_split<PREC, ROWB, BN>(tiles, a.KB);
+  a.split = split > 0 ? usable_split(split, tiles) : auto_split<PREC, ROWB, BN>(tiles, a.KB);
   a.split = std::max(1, std::min(a.split, a.KB));
   if (a.split > 1) {
     if ((long long)tiles * a.split > 0x7fffffffLL) return B200D2_ERR_UNSUPPORTED;
@@ -3851,7 +3858,9 @@ extern "C" int b200d2_plan_create(const b200d2_view* view, const float* d_eulers
   p->var = GemmVariant();
   p->var.row_bytes = g_var_rb.load() > 0 ? g_var_rb.load() : gemm_row_bytes();
   p->var.bn = g_var_bn.load() > 0 ? g_var_bn.load() : 256;
-  p->var.split = g_var_split.load() > 0 ? std::min(g_var_split.load(), kMaxSplit) : 1;
+  p->var.split = g_var_split.load() > 0
+                     ? usable_split(g_var_split.load(), p->var.bn == 128 ? (long long)tiles128.size() : (long long)tiles.size())
+                     : 1;
   p->var.pair = g_var_pair.load() == 1 && p->var.bn == 256 && p->var.split == 1 ? 1 : 2;
   st = plan_pipeline(p, p->stream, p->var);
   if (st == B200D2_OK) st = status_from_cuda(cudaStreamSynchronize(p->stream));

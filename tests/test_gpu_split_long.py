@@ -91,3 +91,29 @@ def test_plan(pkg, cuda, setup, split, tn):
         o = torch.as_tensor(subsets[p], device="cuda").long()
         _check(outs[p], ref[p][o][:, :Ts[p]], "BF16X3")
     plan.close()
+
+
+def test_set_split_does_not_reach_full_grids(pkg, cuda, setup):
+    """A set split is for grids that leave SMs idle: where the tiles fill the GPU
+    none is taken (a plan says so), and the CTA pairs that were asked for run."""
+    torch = cuda
+    pr, view, _, _, _, tx, ty, re, im, corr, _, _ = setup
+    O, T, P = 4608, 113, 30
+    eul = torch.as_tensor(np.ascontiguousarray(pr.eulers.reshape(-1, 9)[:O].reshape(-1)), device="cuda")
+    which = [p % pr.P for p in range(P)]
+    out = torch.empty((P, O, T), device="cuda")
+    parts = [dict(real=re[w], imag=im[w], corr=corr[w], diff2=out[p], orient=None, O=O, trans_x=pr.trans_x[:T].copy(),
+                  trans_y=pr.trans_y[:T].copy()) for p, w in enumerate(which)]
+    pkg.set_gemm_variant(128, 256, 4, 1)
+    try:
+        plan = pkg.Plan(view, eul, O, pr.N_img, parts, precision=pkg.PREC_BF16X3, flags=0)
+        info = plan.info()
+    finally:
+        pkg.set_gemm_variant(0, 0, 0, 0)
+    assert (info["split"], info["pair"]) == (1, 1)
+    plan.run()
+    r = torch.zeros(O * T, device="cuda", dtype=torch.float64)
+    t = [torch.as_tensor(np.ascontiguousarray(a[:T]), device="cuda") for a in (pr.trans_x, pr.trans_y)]
+    pkg.run_diff2_kernel_coarse_double(view, *t, corr[0], re[0], im[0], eul, r, O, T, pr.N_img)
+    _check(out[0].reshape(-1), r, "BF16X3")
+    plan.close()
