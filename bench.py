@@ -1013,8 +1013,10 @@ def ours_arm(args):
                 "single_particle_call": single,
                 "serving": serving,
                 "clocks": clk, "gpu_launches": int(l1 - l0), "kernels": kern.get("per_kernel_ms"),
-                "kernels_note": "each stage timed alone (CUDA events, 3 launches); stages 1, 3 and 5 overlap "
-                                "stages 2 and 4 on a side stream inside a step, so their sum exceeds ms_per_step"}
+                "kernels_note": "each stage that launches anything, timed alone (CUDA events, 3 launches); inside a "
+                                "step the phase tables and the operand generation (and the images' norms, where the "
+                                "projections and theirs are separate kernels) overlap the projections and norms on a "
+                                "side stream, so the sum exceeds ms_per_step"}
         print(json.dumps(line), flush=True)
     proj.close()
     if dist:

@@ -677,6 +677,8 @@ def stage_names(precision: int) -> list[str]:
 
 def kernel_breakdown(view: View, batch: Batch, precision: int, workspace=None, stream=None, reps: int = 3) -> dict:
     """Time each pipeline stage (one kernel each) with CUDA events on `stream`.
+    A stage that launches nothing for this batch (projections that a later stage
+    takes along, minima that no one asked for) is left out.
 
     Runs every stage in order `reps` times (the outputs accumulate; callers
     reset them afterwards if they need the values)."""
@@ -685,9 +687,10 @@ def kernel_breakdown(view: View, batch: Batch, precision: int, workspace=None, s
     names = stage_names(precision)
     ws = _ptr(workspace) if workspace is not None else None
     nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    acc = {n: 0.0 for n in names}
+    acc = {}
     for _ in range(reps):
         for i, n in enumerate(names):
+            launched = launch_count()
             a = torch.cuda.Event(enable_timing=True)
             b = torch.cuda.Event(enable_timing=True)
             a.record(st)
@@ -695,7 +698,8 @@ def kernel_breakdown(view: View, batch: Batch, precision: int, workspace=None, s
                                                          _stream(st)), "batch_stage")
             b.record(st)
             b.synchronize()
-            acc[n] += a.elapsed_time(b)
+            if launch_count() > launched:
+                acc[n] = acc.get(n, 0.0) + a.elapsed_time(b)
     per = {n: v / reps for n, v in acc.items()}
     dom = max(per, key=per.get) if per else None
     return {"per_kernel_ms": per, "dominant": dom, "dominant_ms": per.get(dom) if dom else None, "traffic": None}
