@@ -33,12 +33,12 @@
 //  * the next chunk's texture fetches and shifted images are produced while
 //    the current one is summed (two buffers, one barrier a chunk); its pixels
 //    are copied to shared memory a chunk ahead of that.
-// Bound: the FP32 pipe.  4608 x 113 samples of one particle at image 64: 95 us
-// for 4 lane operations per (o, t, pixel) at 128 a clock and SM, 107 with the
-// tile's 128 translations; 191 us here (the sums' and the staging's
-// instructions together fill the issue slots: a packed instruction takes two),
-// 449 us with a 32-orientation
-// tile per CTA, a sincosf per (pixel, translation, tile) and 5 operations.
+// Bound: the FP32 pipe and its operands.  4608 x 113 samples of one particle at
+// image 64: 95 us for 4 lane operations per (o, t, pixel) at 128 a clock and SM,
+// 107 with the tile's 128 translations; 188 us here (issue slots 55 % busy, the
+// shared-memory and texture path 56 %, 16 warps a SM), 449 us with a
+// 32-orientation tile per CTA, a sincosf per (pixel, translation, tile) and 5
+// operations.
 //
 // The CC form (cuda_kernel_diff2_CC_coarse, src/diff2.cuh:691-809) runs the
 // same tiles with S scaled by corr and A plain: two multiply-adds per
