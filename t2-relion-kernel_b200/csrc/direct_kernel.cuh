@@ -259,6 +259,9 @@ __global__ void __launch_bounds__(NT, dir_min_ctas(NT)) diff2_direct_kernel(cons
   const float* __restrict__ g_im = a.im + p * a.img_stride;
   const float* __restrict__ g_corr = a.corr + p * a.img_stride;
 
+  constexpr bool kScaled = !CC && std::is_same<E, float>::value;
+  __shared__ float s_x2[2][KC];  // kScaled: sum corr/2 |X|^2 of the scaled pixels (even and odd chunks)
+  if (kScaled && tid < 2 * KC) s_x2[tid / KC][tid % KC] = 0.f;
   for (int i = tid; i < BO * 6; i += NT) {
     const int o = o0 + i / 6, c = i % 6;
     const int src = (c >> 1) * 3 + (c & 1);  // e0 e1 e3 e4 e6 e7
@@ -367,10 +370,7 @@ __global__ void __launch_bounds__(NT, dir_min_ctas(NT)) diff2_direct_kernel(cons
   const int nchunk = (ke - kb + KC - 1) / KC;
   // FP32 diff2 scales A and S by sqrt(corr/2) before it subtracts them; `plain`
   // takes the differences first and leaves the weights to the sums
-  constexpr bool kScaled = !CC && std::is_same<E, float>::value;
   bool plain = false;
-  __shared__ float s_x2[2][KC];  // sum corr/2 |X|^2 of the scaled pixels (even and odd chunks)
-  if (kScaled && tid < 2 * KC) s_x2[tid / KC][tid % KC] = 0.f;
   // Pixels of a chunk into slot c % 3, by the first lanes of warp c % (NT / 32):
   // their places and loads first (into shared memory: registers are short here),
   // the values a chunk later, when they have landed.
