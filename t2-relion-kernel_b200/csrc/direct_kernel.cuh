@@ -41,12 +41,12 @@
 // operations.
 //
 // The CC form (cuda_kernel_diff2_CC_coarse, src/diff2.cuh:691-809) runs the
-// same tiles with S scaled by corr and A plain: two multiply-adds per
+// same tiles with S scaled by corr and A plain: one packed multiply-add per
 // (o, t, pixel) for sum corr Re(conj(A) S); the output is -cross / sqrt(norm),
 // written (or added with accumulate).  Pixels outside the projector radius have
 // A = 0 and are skipped.  sum corr |A|^2 is added up by the threads that stage
 // A: in the tile it was repeated by every translation's lanes and its registers
-// spilled (64 particles x 4608 x 113: 17.5 ms, now 8.4).
+// spilled (64 particles x 4608 x 113: 17.5 ms, now 6.7).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -145,15 +145,15 @@ __device__ __forceinline__ void copy_async(float* dst, const float* src) {
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The sums of one (orientation, translation) over the pixels.
-//  FP32 diff2: the pair of its squares, with A and S scaled by sqrt(corr/2)
-//    (mac), or the weight in the sum (weighted).
-//  FP64 diff2: the weight is in the sum.
-//  CC: one sum; S carries corr.
+//  FP32: the pair of the real and the imaginary parts' sums.  diff2 scales A and
+//    S by sqrt(corr/2) (mac of the difference with itself) or leaves the weight
+//    to the sum (weighted); CC's S carries corr (mac).
+//  FP64: one sum; diff2 with the weight in it.
 template <class PR, bool CC>
 struct Acc {
   typename PR::E v;
   __device__ __forceinline__ void clear() { v = 0; }
-  __device__ __forceinline__ void mac(typename PR::V a, typename PR::V b) {  // CC: a, b; diff2: not used
+  __device__ __forceinline__ void mac(typename PR::V a, typename PR::V b) {
     typename PR::E ax, ay, bx, by;
     PR::parts(a, ax, ay);
     PR::parts(b, bx, by);
@@ -166,8 +166,8 @@ struct Acc {
   }
   __device__ __forceinline__ typename PR::E total() const { return v; }
 };
-template <>
-struct Acc<PairF, false> {
+template <bool CC>
+struct Acc<PairF, CC> {
   PairF::V v;
   __device__ __forceinline__ void clear() { v = PairF::zero(); }
   __device__ __forceinline__ void mac(PairF::V a, PairF::V b) { v = PairF::fma(a, b, v); }
